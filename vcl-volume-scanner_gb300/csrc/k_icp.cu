@@ -4,29 +4,25 @@
 // :790-1042) launches one kernel per iteration, copies 1200 x 42 block
 // partial sums to the host, adds them serially in FP32, solves the 6x6 system
 // with an FP32 Cholesky on the host and copies the new increment back: three
-// blocking transfers per iteration.  Here one launch per iteration does it
-// all:
+// blocking transfers per iteration.  Here one launch does every iteration:
 //   per pixel   FP32 Jacobian row A (6) and residual b (d_cssfp, :279-395)
 //   per thread  accumulation of the 27 unique sums (21 of ATA, 6 of ATb)
 //               plus count and sum b^2, in the configured precision
 //   per block   warp-shuffle butterfly, then shared memory across warps
-//   per grid    single pass: the last block to finish (atomic ticket) sums
+//   per grid    the last block to finish an iteration (atomic ticket) sums
 //               the block partials in a fixed order, solves the 6x6 system in
-//               FP64 (Cholesky LL^T with the reference's failure rules,
+//               FP64 (LDL^T with the reference's failure rules,
 //               _yooji_cuda_math.h:489-592), tests convergence
 //               (|x|_inf < 5e-7, :971-972) and applies the SE(3) update in
 //               FP64 (T_12 <- exp(x) T_12, :976-978)
-// Convergence and failure are flags in device memory that the following
-// launches read first, so a whole frame of iterations is one CUDA graph with
-// no host round trip.  Nothing in these kernels waits on another block.
 //
-// Batches: one launch per iteration serves every session of a batch table.
-// A session at level l owns icp_blocks(W_l H_l) block ranges ("virtual
-// blocks"), laid out as they would be in a grid of that size; the persistent
-// grid walks the ranges of all sessions, each session has its own partial
-// buffer and arrival counter, and the range that arrives last for a session
-// reduces and solves that session's system.  Sums therefore run in the same
-// order whatever else shares the launch.
+// Batches: the launch serves every session of a batch table.  A session at
+// level l owns icp_blocks(W_l H_l) block ranges ("virtual blocks"), laid out
+// as they would be in a grid of that size; the persistent grid's blocks claim
+// ranges of any session, each session has its own partial buffer and arrival
+// counter, and the range that arrives last for a session reduces and solves
+// that session's system.  Sums therefore run in the same order whatever else
+// shares the launch.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -424,13 +420,14 @@ __device__ double warp_se3_exp(double x, int lane) {
   return q[3 + r] + B * wxv[r] + C * (q[r] * wv - th2 * q[3 + r]);
 }
 
-// out = A * B (4x4, lane l < 16 computes element l); A in shared memory
+// out = A * B (4x4, lane l < 16 computes element l); A in shared memory, B in
+// global memory, read from L2 (another block of the launch may have written it)
 __device__ void warp_compose(const double* A, const double* B, double* out, int lane) {
   if (lane < 16) {
     const int r = lane >> 2, c = lane & 3;
     double s = 0.0;
 #pragma unroll
-    for (int k = 0; k < 4; k++) s += A[r * 4 + k] * B[k * 4 + c];
+    for (int k = 0; k < 4; k++) s += A[r * 4 + k] * __ldcg(B + k * 4 + c);
     out[lane] = s;
   }
   __syncwarp();
@@ -460,114 +457,229 @@ __device__ void warp_compose_and_invert(const double* E, double* T12, double* Tn
     T21_out[lane] = (float)ti;
   }
 }
-// single-thread inverse used once per frame by k_icp_begin
-__device__ void rigid_inverse(const double* T, double* I) {
-  for (int i = 0; i < 3; i++)
-    for (int j = 0; j < 3; j++) I[i * 4 + j] = T[j * 4 + i];
-  for (int i = 0; i < 3; i++) I[i * 4 + 3] = -(T[0 * 4 + i] * T[3] + T[1 * 4 + i] * T[7] + T[2 * 4 + i] * T[11]);
-  I[12] = I[13] = I[14] = 0.0;
-  I[15] = 1.0;
+// ---- scheduling: one persistent launch for every iteration of every session
+//
+// words[slot] is a session's work word: [31:30] the pyramid level its current
+// iteration runs at (kWordDone: no iteration left), [29:16] the iterations
+// finished at that level, [15:0] the next range of the current iteration.  A
+// block claims a range with one atomicAdd on the word; the block whose range
+// arrives last closes the iteration (sums, solve, pose update) and publishes
+// the next one by storing a new word.  Sessions therefore move through their
+// iterations independently: while one is being closed, the blocks work on
+// another's ranges, and an iteration that a session does not need (it
+// converged) costs nothing.  With one launch per iteration every iteration
+// paid the launch, the reads of the tables and the slowest session's closing
+// block: tracking of one 640x480 frame took 307 us in 19 launches and takes
+// 242 us here, with FP64 sums 603 and 440 us; a 640x480 frame 611 -> 545 us, a
+// 320x240 frame 477 -> 427 us.
+//
+// Progress needs no block but the running ones: a range is claimed only by a
+// block that then runs it, a closer goes on claiming ranges itself, and a
+// block that finds nothing to claim holds nothing, so it may leave at any
+// time.  It leaves when every session is done, or when the unfinished
+// sessions could not give it a range (blocks are numbered, and the block's
+// number is not below the sum of their largest range counts), which frees its
+// SM for other streams' kernels.
+constexpr unsigned kWordDone = 3u;
+constexpr int kIdleLimit = 1 << 22;  // looks without a range before a block gives up (seconds; none in a sound run)
+
+__device__ __forceinline__ unsigned work_word(int level, int iter) {
+  return ((unsigned)level << 30) | ((unsigned)iter << 16);
+}
+__device__ __forceinline__ unsigned load_word(const unsigned* p) { return *(const volatile unsigned*)p; }
+
+// the session's next level with iterations, from l down; -1: none
+__device__ inline int next_level(const SessionDev* s, int l) {
+  while (l >= 0 && s->iters[l] <= 0) l--;
+  return l;
 }
 
-__global__ void k_icp_begin(const BatchTable* __restrict__ bt, int allow_skip, int with_init,
+// end of a session's tracking, one warp: T_gc <- T12 T_gc unless it failed
+// or was skipped
+__device__ void icp_finish(Pose* P, bool skip, bool failed, int frame_mode, int ln, double* Tn, double* A) {
+  if (!skip && !failed) {
+    if (ln < 16) A[ln] = __ldcg(&P->T12[ln]);
+    __syncwarp();
+    double Ti;
+    warp_compose(A, P->T_gc, Tn, ln);
+    if (ln < 16) P->T_gc[ln] = Tn[ln];
+    warp_rigid_inverse(Tn, ln, Ti);
+    if (ln < 16) {
+      P->Tgc[ln] = (float)Tn[ln];
+      P->Tcg[ln] = (float)Ti;
+    }
+    if (ln == 3 || ln == 7 || ln == 11) P->center[ln >> 2] = (float)Ti;
+  }
+  if (ln == 0) {
+    P->tracked = failed ? 0 : 1;
+    if (frame_mode) P->frame += 1;
+  }
+}
+
+// one warp per slot: the increment of this frame starts at identity (or at
+// `init`, and then only level 0 runs), and the session's first iteration is
+// published
+__global__ void k_icp_begin(const BatchTable* __restrict__ bt, unsigned* words, int frame_mode, int with_init,
                             const float* init) {
-  const int i = threadIdx.x;
-  if (i >= bt->n) return;
-  Pose* P = bt->s[i]->pose;
-  P->skip = (allow_skip && P->frame == 0) ? 1 : 0;
-  P->failed = 0;
-  P->iters_run = 0;
-  P->valid_count = 0;
-  for (int l = 0; l < kMaxLevels; l++) P->level_done[l] = (with_init && l > 0) ? 1 : 0;
-  double T[16];
-  for (int k = 0; k < 16; k++) T[k] = (k % 5 == 0) ? 1.0 : 0.0;
-  if (with_init && init)
-    for (int k = 0; k < 16; k++) T[k] = (double)init[k];
-  double I[16];
-  rigid_inverse(T, I);
-  for (int k = 0; k < 16; k++) {
-    P->T12[k] = T[k];
-    P->T21[k] = (float)I[k];
+  if ((int)blockIdx.x >= bt->n) return;
+  const SessionDev* s = bt->s[blockIdx.x];
+  Pose* P = s->pose;
+  const int ln = threadIdx.x;
+  __shared__ double T[16], Tn[16], A[16];
+  const bool skip = frame_mode && P->frame == 0;
+  if (ln < 16) T[ln] = (with_init && init) ? (double)init[ln] : ((ln % 5 == 0) ? 1.0 : 0.0);
+  __syncwarp();
+  double Ti;
+  warp_rigid_inverse(T, ln, Ti);
+  if (ln < 16) {
+    P->T12[ln] = T[ln];
+    P->T21[ln] = (float)Ti;
+  }
+  const int l = skip ? -1 : next_level(s, with_init ? 0 : s->levels - 1);
+  __syncwarp();
+  if (l < 0) icp_finish(P, skip, false, frame_mode, ln, Tn, A);
+  if (ln == 0) {
+    P->skip = skip ? 1 : 0;
+    P->failed = 0;
+    P->iters_run = 0;
+    P->valid_count = 0;
+    *s->icp_counter = 0u;
+    words[blockIdx.x] = l < 0 ? kWordDone << 30 : work_word(l, 0);
   }
 }
 
 // warp 0 of the block that closed a session's iteration: FP64 solve and SE(3)
 // update, lane-parallel (kept out of line so the pixel loop's register
-// allocation does not carry it)
-__device__ __noinline__ void icp_solve_update(Pose* P, const double* fin, int level) {
+// allocation does not carry it).  Returns the session's next work word.
+__device__ __noinline__ unsigned icp_solve_update(const SessionDev* s, const double* fin, int level, int iter,
+                                                  int frame_mode) {
+  __shared__ double E[16], Tn[16];
+  Pose* P = s->pose;
   const int ln = threadIdx.x;
   if (ln < 29) P->last_sums[ln] = fin[ln];
   if (ln == 0) {
-    P->iters_run += 1;
+    atomicAdd(&P->iters_run, 1);
     P->valid_count = (int)fin[27];
   }
   double x;
   const int st = warp_solve6(fin, ln, x);
-  if (st == 1) {
-    if (ln == 0) P->failed = 1;
-    return;
+  bool done = st == 1;
+  if (st != 1) {
+    if (ln < 6) P->last_x[ln] = (float)x;
+    // |x|_inf < 5e-7 ends the level (d_niv_Norm_Infinity_Vector: NaN entries never
+    // raise the maximum, so an all-NaN solution also ends it)
+    const bool big = (ln < 6) && (fabs(x) >= 5.0e-7);
+    const bool ends = st == 2 || !__any_sync(0xffffffffu, big);
+    if (!ends) {
+      const double e = warp_se3_exp(x, ln);
+      if (ln < 16) E[ln] = e;
+      __syncwarp();
+      warp_compose_and_invert(E, P->T12, Tn, ln, P->T12, P->T21);
+      __syncwarp();
+    }
+    if (!ends && iter + 1 < s->iters[level]) return work_word(level, iter + 1);
+    const int l = next_level(s, level - 1);
+    if (l >= 0) return work_word(l, 0);
+  } else if (ln == 0) {
+    P->failed = 1;
   }
-  if (ln < 6) P->last_x[ln] = (float)x;
-  // |x|_inf < 5e-7 ends the level (d_niv_Norm_Infinity_Vector: NaN entries never
-  // raise the maximum, so an all-NaN solution also ends it)
-  const bool big = (ln < 6) && (fabs(x) >= 5.0e-7);
-  if (st == 2 || !__any_sync(0xffffffffu, big)) {
-    if (ln == 0) P->level_done[level] = 1;
-    return;
-  }
-  __shared__ double E[16], Tn[16];
-  const double e = warp_se3_exp(x, ln);
-  if (ln < 16) E[ln] = e;
-  __syncwarp();
-  warp_compose_and_invert(E, P->T12, Tn, ln, P->T12, P->T21);
-  __syncwarp();
+  icp_finish(P, false, done, frame_mode, ln, Tn, E);
+  return kWordDone << 30;
 }
 
-// Blocks take ranges from an atomic counter: a block that closes a session
-// (reduction + solve, ~10 us) simply takes no new range meanwhile, so the
-// closing work of different sessions overlaps instead of queueing behind a
-// static assignment.  The last block to leave clears the counters.
 #ifndef VS_ICP_MIN_BLOCKS
 #define VS_ICP_MIN_BLOCKS 3  // resident 256-thread blocks per SM the register allocation must allow
 #endif
 
+// One warp claims a range: *out_slot its session (-1: leave), *out_word the
+// session's word with the range.  The block stays with the session it worked
+// on (prefer) while that has ranges; otherwise it takes the first session that
+// does, so that few sessions are under way at a time and their maps stay in
+// L2 over their iterations.
+__device__ __noinline__ void claim_range(unsigned* __restrict__ words, int n, const SessionDev* const* sS,
+                                         const int (*sNvb)[kMaxSlots], int prefer, int* out_slot,
+                                         unsigned* out_word) {
+  const int lane = threadIdx.x & 31;
+  int slot = -1;
+  unsigned w = 0u;
+  auto available = [&](int q, unsigned v) { return (int)(v & 0xffffu) < sNvb[v >> 30][q]; };
+  for (int look = 0;; look++) {
+    int first = prefer;
+    if (first < 0) {
+      int need = 0;
+#pragma unroll
+      for (int h = 0; h < kMaxSlots; h += 32) {
+        const int q = h + lane;
+        const unsigned v = q < n ? load_word(words + q) : kWordDone << 30;
+        const unsigned m = __ballot_sync(0xffffffffu, available(q, v));
+        if (m && first < 0) first = h + __ffs(m) - 1;
+        if ((v >> 30) != kWordDone) need += max(sNvb[0][q], max(sNvb[1][q], sNvb[2][q]));
+      }
+      need = __reduce_add_sync(0xffffffffu, need);
+      if (first < 0) {
+        if ((int)blockIdx.x >= need) break;
+        if (look >= kIdleLimit) {
+          // an iteration that does not end: its frame counts as lost
+          for (int q = lane; q < n; q += 32)
+            if ((load_word(words + q) >> 30) != kWordDone) sS[q]->pose->failed = 1, sS[q]->pose->tracked = 0;
+          break;
+        }
+        __nanosleep(40);
+        continue;
+      }
+    }
+    if (lane == 0) w = atomicAdd(words + first, 1u);
+    w = __shfl_sync(0xffffffffu, w, 0);
+    if (available(first, w)) {
+      slot = first;
+      break;
+    }
+    prefer = -1;  // no range left there, or another block was faster
+  }
+  if (lane == 0) {
+    *out_slot = slot;
+    *out_word = w;
+  }
+  __threadfence();  // the session's pose is read after its word
+}
+
 template <int MODE>
 __global__ void __launch_bounds__(kThreads, VS_ICP_MIN_BLOCKS)
-    k_icp_iter(const BatchTable* __restrict__ bt, unsigned* __restrict__ work, int level, int iter) {
+    k_icp_run(const BatchTable* __restrict__ bt, unsigned* __restrict__ words, int frame_mode) {
   typedef typename PartT<MODE>::type PT;
   __shared__ PT wsum[kThreads / 32][29];
-  __shared__ int s_last, s_item;
   __shared__ double fin[29];
   __shared__ float sT21[12], sK[4];
+  __shared__ const SessionDev* sS[kMaxSlots];
+  __shared__ int sNvb[4][kMaxSlots];  // ranges of an iteration at level 0..2 (0: no such level); [3]: none (done)
+  __shared__ int s_slot, s_close;
+  __shared__ unsigned s_word;
   const int n = bt->n;
-  const int* pre = bt->icp[level];
-  const int total = pre[n];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (;;) {
-    if (threadIdx.x == 0) s_item = (int)atomicAdd(work, 1u);
-    __syncthreads();
-    const int item = s_item;
-    if (item >= total) break;
-    int vb;
-    const int slot = find_slot(pre, n, item, vb);
-    const SessionDev* __restrict__ s = bt->s[slot];
-    Pose* P = s->pose;
-    // uniform across the session's ranges: no range of this session has
-    // closed the iteration yet when any of them reads the flags
-    if (iter >= s->iters[level] || (P->skip | P->failed | P->level_done[level])) {
-      // the session sits this launch out (its flags do not change during the
-      // launch): move the counter past its remaining ranges at once
-      if (threadIdx.x == 0) atomicMax(work, (unsigned)pre[slot + 1]);
-      __syncthreads();  // every thread has read s_item before the next fetch
-      continue;
-    }
-    const int nvb = pre[slot + 1] - pre[slot];
+  if (threadIdx.x < kMaxSlots) {
+    const int i = threadIdx.x;
+    sS[i] = i < n ? bt->s[i] : nullptr;
+#pragma unroll
+    for (int l = 0; l < kMaxLevels; l++) sNvb[l][i] = i < n ? bt->icp[l][i + 1] - bt->icp[l][i] : 0;
+    sNvb[kMaxLevels][i] = 0;
+  }
+  __syncthreads();
+
+  auto claim = [&](int prefer) { claim_range(words, n, sS, sNvb, prefer, &s_slot, &s_word); };
+  if (warp == 0) claim(-1);
+  __syncthreads();
+  while (s_slot >= 0) {
+    const int slot = s_slot;
+    const unsigned word = s_word;
+    const int level = (int)(word >> 30), iter = (int)((word >> 16) & 0x3fffu), vb = (int)(word & 0xffffu);
+    const int nvb = sNvb[level][slot];
+    const SessionDev* __restrict__ s = sS[slot];
     const int w = s->lv[level].W, h = s->lv[level].H;
     // the pose and intrinsics are read from shared memory in the pixel loop,
-    // which leaves the registers to the 29 running sums
-    if (threadIdx.x < 12) sT21[threadIdx.x] = P->T21[threadIdx.x];
-    if (threadIdx.x < 4) sK[threadIdx.x] = s->lv[level].K[threadIdx.x];
-    __syncthreads();
+    // which leaves the registers to the 29 running sums; the pose comes from
+    // L2 (this SM's L1 may hold an earlier iteration's)
+    if (threadIdx.x < 12) sT21[threadIdx.x] = __ldcg(&s->pose->T21[threadIdx.x]);
+    if (threadIdx.x >= 32 && threadIdx.x < 36) sK[threadIdx.x - 32] = s->lv[level].K[threadIdx.x - 32];
     const float* K = sK;
     const float* T21 = sT21;
     const float th = s->th_icp, cosn = s->cos_normal;
@@ -590,6 +702,7 @@ __global__ void __launch_bounds__(kThreads, VS_ICP_MIN_BLOCKS)
       d_next = __ldg(depth + p);
       if (ntest) q_next = __ldg(innrm + p);
     }
+    __syncthreads();
     while (p < npix) {
       const float d1 = d_next;
       const float4 qn = q_next;
@@ -613,21 +726,24 @@ __global__ void __launch_bounds__(kThreads, VS_ICP_MIN_BLOCKS)
     const PT mine = acc.reduce_scatter(lane);
     if (lane < 29) wsum[warp][lane] = mine;
     __syncthreads();
-    PT* part = reinterpret_cast<PT*>(s->partials) + (size_t)vb * kPartials;
-    if (threadIdx.x < 29) {
-      PT v = wsum[0][threadIdx.x];
-      for (int q = 1; q < kThreads / 32; q++) v = combine(v, wsum[q][threadIdx.x], MODE);
-      part[threadIdx.x] = v;
-      __threadfence();
+    if (warp == 0) {
+      if (lane < 29) {
+        PT v = wsum[0][lane];
+        for (int q = 1; q < kThreads / 32; q++) v = combine(v, wsum[q][lane], MODE);
+        reinterpret_cast<PT*>(s->partials)[(size_t)vb * kPartials + lane] = v;
+        __threadfence();
+      }
+      __syncwarp();
+      unsigned t = 0u;
+      if (lane == 0) t = atomicAdd(s->icp_counter, 1u);
+      t = __shfl_sync(0xffffffffu, t, 0);
+      const bool last = t == (unsigned)nvb - 1u;
+      if (lane == 0) s_close = last;
+      if (!last) claim(slot);
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-      unsigned t = atomicAdd(s->icp_counter, 1u);
-      s_last = (t == (unsigned)nvb - 1u);
-    }
-    __syncthreads();
-    if (s_last) {
-      // ---- last range of this session: deterministic sum, then the solve ----
+    if (s_close) {
+      // ---- last range of this iteration: deterministic sum, then the solve ----
       __threadfence();
       {
         // 8 threads per quantity, each a fixed stride over the ranges, then a
@@ -637,20 +753,20 @@ __global__ void __launch_bounds__(kThreads, VS_ICP_MIN_BLOCKS)
         v.x = 0;
         v.y = 0;
         if (k < 29) {
-          // four partials in flight per thread, combined in the same order
+          // eight partials in flight per thread, combined in the same order
           // as one at a time (a missing one combines as an exact zero)
           const PT* base = reinterpret_cast<const PT*>(s->partials);
-          for (int bb = j; bb < nvb; bb += 32) {
-            PT t4[4];
+          for (int bb = j; bb < nvb; bb += 64) {
+            PT t8[8];
 #pragma unroll
-            for (int u = 0; u < 4; u++) {
+            for (int u = 0; u < 8; u++) {
               const int q = bb + 8 * u;
-              t4[u].x = 0;
-              t4[u].y = 0;
-              if (q < nvb) t4[u] = __ldcg(base + (size_t)q * kPartials + k);
+              t8[u].x = 0;
+              t8[u].y = 0;
+              if (q < nvb) t8[u] = __ldcg(base + (size_t)q * kPartials + k);
             }
 #pragma unroll
-            for (int u = 0; u < 4; u++) v = combine(v, t4[u], MODE);
+            for (int u = 0; u < 8; u++) v = combine(v, t8[u], MODE);
           }
         }
 #pragma unroll
@@ -658,45 +774,16 @@ __global__ void __launch_bounds__(kThreads, VS_ICP_MIN_BLOCKS)
         if (k < 29 && j == 0) fin[k] = (double)v.x + (double)v.y;
       }
       __syncthreads();
-      if (threadIdx.x < 32) {
-        if (threadIdx.x == 0) *s->icp_counter = 0u;
-        icp_solve_update(P, fin, level);
+      if (warp == 0) {
+        const unsigned next = icp_solve_update(s, fin, level, iter, frame_mode);
+        if (lane == 0) *s->icp_counter = 0u;
+        __threadfence();  // every lane's pose writes, then the word
+        __syncwarp();
+        if (lane == 0) atomicExch(words + slot, next);
+        claim((next >> 30) == kWordDone ? -1 : slot);
       }
+      __syncthreads();
     }
-    __syncthreads();  // shared sums and s_item are reused by the next range
-  }
-  if (threadIdx.x == 0) {
-    __threadfence();
-    if (atomicAdd(work + 1, 1u) == gridDim.x - 1) {
-      work[0] = 0u;
-      work[1] = 0u;
-      __threadfence();
-    }
-  }
-}
-
-// one warp per slot
-__global__ void k_icp_finish(const BatchTable* __restrict__ bt, int frame_mode) {
-  if ((int)blockIdx.x >= bt->n) return;
-  Pose* P = bt->s[blockIdx.x]->pose;
-  const int ln = threadIdx.x;
-  __shared__ double Tn[16], A[16];
-  if (!P->skip && !P->failed) {
-    if (ln < 16) A[ln] = P->T12[ln];
-    __syncwarp();
-    double Ti;
-    warp_compose(A, P->T_gc, Tn, ln);
-    if (ln < 16) P->T_gc[ln] = Tn[ln];
-    warp_rigid_inverse(Tn, ln, Ti);
-    if (ln < 16) {
-      P->Tgc[ln] = (float)Tn[ln];
-      P->Tcg[ln] = (float)Ti;
-    }
-    if (ln == 3 || ln == 7 || ln == 11) P->center[ln >> 2] = (float)Ti;
-  }
-  if (ln == 0) {
-    P->tracked = P->skip ? 1 : (P->failed ? 0 : 1);
-    if (frame_mode) P->frame += 1;
   }
 }
 
@@ -751,31 +838,30 @@ int icp_blocks(int npix, int level) {
   return b;
 }
 
-void launch_icp(const BatchTable* bt, int max_levels, const int* max_iters, int reduce_mode, cudaStream_t st,
-                bool frame_mode, const float* init_T12) {
+void launch_icp(const BatchTable* bt, int reduce_mode, cudaStream_t st, bool frame_mode, const float* init_T12) {
   // frame-level calls skip tracking on the first frame as so_Scan_Object does
   // (zz_flag_track, z_yooji_object_scanner.cpp:534,572-576); explicit
   // tp_Track_Pose calls always track
-  const bool with_init = init_T12 != nullptr;
-  k_icp_begin<<<1, kMaxSlots, 0, st>>>(bt, frame_mode ? 1 : 0, with_init ? 1 : 0, init_T12);
-  const int grid = sm_count() * VS_ICP_MIN_BLOCKS;  // every block resident
-  unsigned* work = const_cast<unsigned*>(bt->work) + 2;
-  for (int l = max_levels - 1; l >= 0; l--) {
-    for (int i = 0; i < max_iters[l]; i++) {
-      switch (reduce_mode) {
-        case VS_REDUCE_FP32:
-          k_icp_iter<VS_REDUCE_FP32><<<grid, kThreads, 0, st>>>(bt, work, l, i);
-          break;
-        case VS_REDUCE_FP64:
-          k_icp_iter<VS_REDUCE_FP64><<<grid, kThreads, 0, st>>>(bt, work, l, i);
-          break;
-        default:
-          k_icp_iter<VS_REDUCE_KAHAN><<<grid, kThreads, 0, st>>>(bt, work, l, i);
-          break;
-      }
-    }
+  unsigned* words = const_cast<unsigned*>(bt->icp_word);
+  const int fm = frame_mode ? 1 : 0;
+  k_icp_begin<<<kMaxSlots, 32, 0, st>>>(bt, words, fm, init_T12 ? 1 : 0, init_T12);
+  // Two of the three blocks that fit an SM: the rest of each SM takes the
+  // other branch's kernels while this launch waits for a closer.  (Sixteen
+  // sessions, two branches: 1955 us per step with three blocks, 1894 with
+  // two, 1922 with one and a half; 64 sessions 5990, 5970, 5925; one session
+  // the same.)
+  const int grid = sm_count() * 2;
+  switch (reduce_mode) {
+    case VS_REDUCE_FP32:
+      k_icp_run<VS_REDUCE_FP32><<<grid, kThreads, 0, st>>>(bt, words, fm);
+      break;
+    case VS_REDUCE_FP64:
+      k_icp_run<VS_REDUCE_FP64><<<grid, kThreads, 0, st>>>(bt, words, fm);
+      break;
+    default:
+      k_icp_run<VS_REDUCE_KAHAN><<<grid, kThreads, 0, st>>>(bt, words, fm);
+      break;
   }
-  k_icp_finish<<<kMaxSlots, 32, 0, st>>>(bt, frame_mode ? 1 : 0);
 }
 
 void launch_pose_set(const SessionDev* d, const double* T_gc, cudaStream_t st) {

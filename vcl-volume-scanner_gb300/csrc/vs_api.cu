@@ -203,7 +203,7 @@ void record_frame(vs_session* s, cudaStream_t st) {
   launch_filter(s->tab, st);
   if (h.cos_normal > -2.0f) launch_input_maps(s->tab, st);
   mark(1);
-  launch_icp(s->tab, h.levels, h.iters, h.reduce_mode, st, true, nullptr);
+  launch_icp(s->tab, h.reduce_mode, st, true, nullptr);
   mark(2);
   const bool color = h.col != nullptr;
   launch_integrate(s->tab, h.tsdf_type, nullptr, nullptr, nullptr, true, st, color);
@@ -448,7 +448,7 @@ int vs_bilateral_filter_depth_host(vs_session* s, float* out_host, const float* 
 
 int vs_track_pose(vs_session* s, const float* init_T01_dev, int* tracked) {
   if (!s) return fail(VS_ERR_ARG, "null session");
-  launch_icp(s->tab, s->h.levels, s->h.iters, s->h.reduce_mode, s->stream, false, init_T01_dev);
+  launch_icp(s->tab, s->h.reduce_mode, s->stream, false, init_T01_dev);
   VS_CU(cudaGetLastError());
   VS_CU(cudaMemcpyAsync(s->host_pose, s->h.pose, sizeof(Pose), cudaMemcpyDeviceToHost, s->stream));
   VS_CU(cudaStreamSynchronize(s->stream));
@@ -676,7 +676,7 @@ int vs_stage_filter(vs_session* s, const uint16_t* depth_mm_dev) {
 }
 int vs_stage_track(vs_session* s) {
   if (!s) return fail(VS_ERR_ARG, "null session");
-  launch_icp(s->tab, s->h.levels, s->h.iters, s->h.reduce_mode, s->stream, true, nullptr);
+  launch_icp(s->tab, s->h.reduce_mode, s->stream, true, nullptr);
   VS_CU(cudaGetLastError());
   return VS_OK;
 }
@@ -874,12 +874,11 @@ int vs_get_frame_stats(vs_session* s, uint32_t* stats) {
 
 int vs_kernels_per_frame(const vs_config* c) {
   if (check_config(c) != VS_OK) return -1;
-  int n = 1 + (c->levels - 1);              // bilateral + pyramid levels
+  int n = 1 + (kMaxLevels - 1);             // bilateral + pyramid levels
   if (c->cos_normal > -2.0f) n += 3;        // input maps: pre, row scan, post
-  n += 2;                                   // ICP begin / finish
-  for (int l = 0; l < c->levels; l++) n += c->icp_iters[l];
+  n += 2;                                   // ICP begin, every iteration
   n += 3;                                   // counter reset, activation, update
-  n += 2;                                   // ray march + shading of every level
+  n += 2 + (c->color ? 2 : 1);              // band distances; ray march and shading of every level
   return n;
 }
 

@@ -12,19 +12,17 @@
 // The sessions are split into kIcpGroups groups (by pixel count), and each
 // group's whole frame (filter, maps, ICP, integration, ray-cast) runs as its
 // own launch sequence on a branch of the graph.  Every persistent launch ends
-// with a tail in which a few blocks still run (for ICP: the blocks closing a
-// session's iteration with a reduction and an FP64 solve; for the ray-cast:
-// the last tiles); with several sequences in flight the other sequences'
-// blocks fill the SMs that a tail leaves idle.  A session's work and sums do
+// with a tail in which a few blocks still run (for ICP: the last sessions'
+// iterations; for the ray-cast: the last tiles); with several sequences in
+// flight the other sequences' blocks fill the SMs that a tail leaves idle.  A session's work and sums do
 // not depend on which sessions share its launches, so the split changes no
 // result.  With stage timing on, the stages run one after another over the
 // whole batch (ICP still on branches) so that each stage's time is its own.
 //
-// The graph depends only on the schedule it was captured for: the deepest
-// pyramid and the largest ICP iteration count per level among the sessions,
-// whether any session needs input normal maps, the reduction mode and the
-// TSDF storage.  Sessions with fewer levels or iterations skip the extra
-// launches on the device; a step that needs a longer schedule recaptures.
+// The graph depends only on the schedule it was captured for: whether any
+// session needs input normal maps or keeps colour, the reduction mode and the
+// TSDF storage.  Levels and ICP iterations are each session's own, inside the
+// launches.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -41,8 +39,6 @@ using namespace vs;
 namespace {
 
 struct Schedule {
-  int levels = 0;
-  int iters[kMaxLevels] = {0, 0, 0};
   int inmaps = 0;
   int reduce_mode = -1;
   int tsdf_type = -1;
@@ -50,10 +46,7 @@ struct Schedule {
   int color = 0;  // some session keeps a colour volume
   bool covers(const Schedule& o) const {
     if (o.reduce_mode != reduce_mode || o.tsdf_type != tsdf_type || o.timing != timing) return false;
-    if (o.levels > levels || (o.inmaps && !inmaps) || (o.color && !color)) return false;
-    for (int l = 0; l < kMaxLevels; l++)
-      if (o.iters[l] > iters[l]) return false;
-    return true;
+    return !(o.inmaps && !inmaps) && !(o.color && !color);
   }
 };
 
@@ -100,7 +93,7 @@ void record_chain(vs_batch* b, const BatchTable* t, cudaStream_t st) {
   const Schedule& k = b->sched;
   launch_filter(t, st, b->shape.bil_rows);
   if (k.inmaps) launch_input_maps(t, st);
-  launch_icp(t, k.levels, k.iters, k.reduce_mode, st, true, nullptr);
+  launch_icp(t, k.reduce_mode, st, true, nullptr);
   launch_integrate(t, k.tsdf_type, nullptr, nullptr, nullptr, true, st, k.color != 0, b->shape.integrate_blocks_per_sm);
   launch_raycast(t, k.tsdf_type, -1, nullptr, nullptr, nullptr, 0.0f, 0.0f, -1.0f, true, nullptr, nullptr, nullptr,
                  nullptr, st, b->shape, nullptr, k.color != 0);
@@ -132,9 +125,9 @@ void record_step(vs_batch* b, int r, cudaStream_t st) {
     mark(1);
     cudaEventRecord(b->fork, st);
     for (int g = 1; g < kIcpGroups; g++) cudaStreamWaitEvent(b->side[g], b->fork, 0);
-    launch_icp(b->d_grp, k.levels, k.iters, k.reduce_mode, st, true, nullptr);
+    launch_icp(b->d_grp, k.reduce_mode, st, true, nullptr);
     for (int g = 1; g < kIcpGroups; g++) {
-      launch_icp(b->d_grp + g, k.levels, k.iters, k.reduce_mode, b->side[g], true, nullptr);
+      launch_icp(b->d_grp + g, k.reduce_mode, b->side[g], true, nullptr);
       cudaEventRecord(b->join[g], b->side[g]);
       cudaStreamWaitEvent(st, b->join[g], 0);
     }
@@ -194,9 +187,6 @@ int check_sessions(vs_batch* b, vs_session* const* ss, int n, Schedule& k) {
     } else if (h.reduce_mode != k.reduce_mode || h.tsdf_type != k.tsdf_type) {
       return fail_code(VS_ERR_ARG, "sessions of a batch must share reduce_mode and tsdf_type");
     }
-    if (h.levels > k.levels) k.levels = h.levels;
-    for (int l = 0; l < h.levels; l++)
-      if (h.iters[l] > k.iters[l]) k.iters[l] = h.iters[l];
     if (h.cos_normal > -2.0f) k.inmaps = 1;
     if (h.col) k.color = 1;
   }
@@ -213,10 +203,8 @@ int launch_step(vs_batch* b, vs_session* const* ss, int n, const Schedule& k, cu
     Schedule m = k;
     if (b->exec[0] && b->sched.reduce_mode == k.reduce_mode && b->sched.tsdf_type == k.tsdf_type &&
         b->sched.timing == k.timing) {
-      m.levels = std::max(m.levels, b->sched.levels);
       m.inmaps |= b->sched.inmaps;
       m.color |= b->sched.color;
-      for (int l = 0; l < kMaxLevels; l++) m.iters[l] = std::max(m.iters[l], b->sched.iters[l]);
     }
     // the graphs read both ring buffers: let in-flight steps finish first
     cudaError_t e = cudaStreamSynchronize(b->stream);

@@ -40,7 +40,6 @@ struct Pose {
   float T21[16];       // float inverse of T12, read by the ICP term kernel
   double T_gc[16];     // FP64 master pose, global -> camera
   double T12[16];      // ICP increment of the current frame (camera t0 -> t1)
-  int level_done[kMaxLevels];
   int failed;          // 6x6 system singular this frame
   int skip;            // no tracking this frame (first frame)
   float last_x[6];
@@ -130,8 +129,9 @@ struct BatchTable {
                                        // also copies it into the session's frame buffer); NULL: that buffer
   int slab[kMaxSlots + 1];             // z slabs of bricks (band distance, x and y passes)
   int brow[kMaxSlots + 1];             // y rows of bricks (band distance, z pass)
-  unsigned work[8];                    // work counters ([0..1] ray march, [2..3] ICP, [4..5] ray
-                                       // shading); zero between launches
+  unsigned work[8];                    // work counters ([0..1] ray march, [4..5] ray shading); zero between
+                                       // launches
+  unsigned icp_word[kMaxSlots];        // per slot: level, iteration and next range of its tracking (k_icp.cu)
 };
 
 // slot of work item b (pre: prefix over n slots), or -1 past the last item
@@ -305,10 +305,8 @@ int ray_max_blocks_per_sm(int tsdf_type, bool shade);
 void launch_filter(const BatchTable* bt, cudaStream_t st, int bil_rows = 8);
 void launch_input_maps(const BatchTable* bt, cudaStream_t st);
 void launch_bilateral_float(const SessionDev& h, const float* in, float* out, cudaStream_t st);
-// ICP of every slot; the schedule runs levels max_levels-1 .. 0 with
-// max_iters[l] launches each (slots with fewer levels or iterations skip)
-void launch_icp(const BatchTable* bt, int max_levels, const int* max_iters, int reduce_mode, cudaStream_t st,
-                bool frame_mode, const float* init_T12_dev);
+// ICP of every slot, each session through its own levels and iterations
+void launch_icp(const BatchTable* bt, int reduce_mode, cudaStream_t st, bool frame_mode, const float* init_T12_dev);
 // depth / Tgc / Tcg: explicit inputs of a one-slot table, or NULL for each
 // session's own level-0 depth and pose; color: run the variant that also
 // blends the colour of sessions that keep a colour volume
