@@ -57,3 +57,40 @@ def test_forty_sessions_each_as_alone(gpu):
     finally:
         for s in sessions:
             s.close()
+
+
+@pytest.mark.parametrize("angle", [0.0, 0.02, 0.3])
+@pytest.mark.parametrize("mode", [V.VS_REDUCE_FP32, V.VS_REDUCE_KAHAN, V.VS_REDUCE_FP64])
+def test_one_iteration_solves_and_applies_its_own_system(gpu, angle, mode):
+    """x solves the recorded normal equations and the pose becomes
+    exp(x) init T_gc, for steps on both sides of the exponential's series
+    range (0.1 rad).  x is recorded in float (relative 2^-24) from an FP64
+    solve (relative error below 1e-15 times the condition number)."""
+    import torch
+    from scipy.linalg import expm
+
+    case = helpers.make_case(width=160, height=120, dim=96, size=1.0, frames=2, seed=9, iters=(1, 0, 0), th_icp=0.25,
+                             reduce_mode=mode)
+    c, s_ = np.cos(angle), np.sin(angle)
+    init = np.eye(4, dtype=np.float32)
+    init[:2, :2] = [[c, -s_], [s_, c]]
+    with V.Session(case["cfg"]) as s:
+        s.scan_frame_host(case["depth"][0])
+        T0 = s.pose()[1]
+        s.stage_filter(torch.from_numpy(case["depth"][1].view(np.int16)).cuda().data_ptr())
+        s.sync()
+        assert s.tp_track_pose(torch.from_numpy(init).cuda().data_ptr())
+        T1, (sums, x) = s.pose()[1], s.icp_system()
+    A = np.zeros((6, 6))
+    A[np.triu_indices(6)] = sums[:21]
+    A = A + np.triu(A, 1).T
+    ref = np.linalg.solve(A, sums[21:27])
+    tol = (2.0 ** -24 + 1e-15 * np.linalg.cond(A)) * 2.0
+    assert np.linalg.norm(x - ref) <= tol * np.linalg.norm(ref)
+    w, v = ref[:3], ref[3:]
+    xi = np.zeros((4, 4))
+    xi[:3, :3] = [[0, -w[2], w[1]], [w[2], 0, -w[0]], [-w[1], w[0], 0]]
+    xi[:3, 3] = v
+    want = expm(xi) @ init.astype(np.float64) @ T0
+    assert np.abs(T1 - want).max() <= 1e-12 * np.linalg.cond(A)
+    print(angle, mode, np.linalg.norm(w), np.linalg.cond(A))
