@@ -268,9 +268,8 @@ __device__ inline int tri_index(int i, int j) { return i * 6 - i * (i - 1) / 2 +
 //     multiply-adds.
 // One column per step with a reciprocal and separate products and sums, and one
 // series per lane, took 10.0 us from an iteration's sums to its published
-// pose (6.4 us where the step ended the level); this takes 5.0 (3.8), about
-// half of it operations, the rest the code's first run on the closing SM.  A
-// 640x480 frame went from 545 to 492 us, a 320x240 frame from 427 to 373.
+// pose (6.4 us where the step ended the level); this takes about 4 (3).  A
+// 640x480 frame went from 545 to 486 us, a 320x240 frame from 427 to 367.
 
 // lane -> (row, col) of the lower triangle, row-major: lane = row*(row+1)/2 + col
 __device__ __forceinline__ int low_lane(int r, int c) { return r * (r + 1) / 2 + c; }
@@ -415,14 +414,9 @@ __device__ __forceinline__ bool warp_solve6(const double* fin, int lane, double&
 // C (w (w.v) - th^2 v), A = sin(th)/th, B = (1 - cos(th))/th^2,
 // C = (th - sin(th))/th^3 - the same function, with no division by th.  For
 // th < 0.1 the three coefficients come from their Taylor series in th^2
-// (truncation below 1e-17 relative), lane l the coefficient l mod 3;
+// (truncation below 1e-17 relative), lane l < 3 the l-th (the constants are selected, not read: a read would
+// miss in the closing SM's constant cache);
 // otherwise from sin/cos.  Lane l < 16 returns element l of the 4x4 result.
-__constant__ double kSe3[6][3] = {{1.0, 1.0 / 2, 1.0 / 6},
-                                  {-1.0 / 6, -1.0 / 24, -1.0 / 120},
-                                  {1.0 / 120, 1.0 / 720, 1.0 / 5040},
-                                  {-1.0 / 5040, -1.0 / 40320, -1.0 / 362880},
-                                  {1.0 / 362880, 1.0 / 3628800, 1.0 / 39916800},
-                                  {-1.0 / 39916800, -1.0 / 479001600, -1.0 / 6227020800}};
 __device__ __noinline__ void se3_far(double th2, double* k) {
   const double th = sqrt(th2);
   const double sn = sin(th), cs = cos(th);
@@ -453,10 +447,13 @@ __device__ __forceinline__ double se3_exp(const double q[6], int lane) {
   const double p = fma(-th2, base, qr * (rot ? qc : wv));
   double A, B, C;
   if (th2 < 0.01) {
-    const int g = lane % 3;
-    double k = kSe3[5][g];
-#pragma unroll
-    for (int i = 4; i >= 0; i--) k = fma(k, th2, kSe3[i][g]);
+    const int g = lane & 3;
+    double k = pick(g, -1.0 / 39916800, -1.0 / 479001600, -1.0 / 6227020800);
+    k = fma(k, th2, pick(g, 1.0 / 362880, 1.0 / 3628800, 1.0 / 39916800));
+    k = fma(k, th2, pick(g, -1.0 / 5040, -1.0 / 40320, -1.0 / 362880));
+    k = fma(k, th2, pick(g, 1.0 / 120, 1.0 / 720, 1.0 / 5040));
+    k = fma(k, th2, pick(g, -1.0 / 6, -1.0 / 24, -1.0 / 120));
+    k = fma(k, th2, pick(g, 1.0, 1.0 / 2, 1.0 / 6));
     A = __shfl_sync(M, k, 0), B = __shfl_sync(M, k, 1), C = __shfl_sync(M, k, 2);
   } else {
     double k[3];
@@ -713,8 +710,10 @@ __device__ __noinline__ unsigned close_iteration(const SessionDev* s, int nvb, i
   __syncthreads();
   unsigned next = 0u;
   if (threadIdx.x < 64) next = icp_close(s, fin, level, iter, frame_mode);
-  __threadfence();
-  __syncwarp();
+  if (threadIdx.x < 32) {
+    __syncwarp();
+    __threadfence();
+  }
   return next;
 }
 
@@ -770,8 +769,8 @@ __device__ __noinline__ void claim_range(unsigned* __restrict__ words, int n, co
   if (lane == 0) {
     *out_slot = slot;
     *out_word = w;
+    __threadfence();  // the block reads the session's pose after its word (and the barrier that follows)
   }
-  __threadfence();  // the session's pose is read after its word
 }
 
 // a load that the compiler does not merge with an earlier one
@@ -883,21 +882,22 @@ __global__ void __launch_bounds__(kThreads, VS_ICP_MIN_BLOCKS)
       if (lane == 0) t = atomicAdd(sr->icp_counter, 1u);
       t = __shfl_sync(0xffffffffu, t, 0);
       const bool last = t == (unsigned)ranges - 1u;
-      if (lane == 0) s_close = last;
+      if (lane == 0) {
+        s_close = last;
+        if (last) {
+          __threadfence();  // the block reads the other ranges' partials after the arrivals
+          *sr->icp_counter = 0u;
+        }
+      }
       if (!last) claim(slot);
     }
     __syncthreads();
     if (s_close) {
       // ---- last range of this iteration ----
-      __threadfence();
       const unsigned next =
           close_iteration<MODE>(sr, ranges, (int)(word >> 30), (int)((word >> 16) & 0x3fffu), frame_mode);
       if (warp == 0) {
-        if (lane == 0) {
-          *sr->icp_counter = 0u;
-          __threadfence();
-          atomicExch(words + slot, next);
-        }
+        if (lane == 0) atomicExch(words + slot, next);
         claim((next >> 30) == kWordDone ? -1 : slot);
       }
       __syncthreads();
