@@ -168,18 +168,31 @@ __global__ void __launch_bounds__(256) k_pyramid_batch(const BatchTable* __restr
 //
 // pass 1 (parallel): per interior pixel, code 0 = no normal (an invalid
 //   point among the 5, or |dx|,|dy| < 1e-7), 1 = normal accepted,
-//   2 = normal rejected by the 60 degree test; candidate normals are stored.
-// pass 2 (one warp per level, rows in order): the reference rewrites the
+//   2 = normal rejected by the 60 degree test; accepted normals are stored,
+//   and codes 1 and 2 as bitmasks of 32 pixels per word.
+// pass 2 (one block per level, rows in order): the reference rewrites the
 //   point map in place on a rejection, which blocks the right and lower
 //   neighbours.  With C = code2 & ~R(row above), a row solves
 //   R_j = C_j & ~R_{j-1}: inside each run of C the rejected pixels alternate
 //   starting at the run's first pixel.  Runs are smeared with one addition
 //   per 32-bit word; the words of a row and the rows themselves are swept as
-//   a wavefront across the lanes of the warp.
+//   a wavefront across the lanes of one warp.  The block then counts the
+//   valid normals before each word.
 // pass 3 (parallel): vertex valid = depth > 0 and not rejected; normal valid =
-//   code 1 and neither the left nor the upper neighbour rejected.
+//   code 1 and neither the left nor the upper neighbour rejected: the normals
+//   that are not are overwritten, and the valid ones' pixels are listed in
+//   raster order for the tracker.
 // A session's items cover its levels in order; the per-level tile counts
 // follow from the level sizes.
+//
+// Passes 1 and 3 are bound by instruction issue and by their writes (16 B
+// normal and 16 B vertex per pixel, each written once but for the normals
+// that pass 3 takes back; 32-row tiles spread the table search of a tile over
+// four rows per thread), pass 2 by the wavefront's chain (about 80 cycles per
+// row; 24 us for 640x480 with the counting, 37 before).  Before, pass 1 wrote
+// candidate normals and a code byte that pass 3 read and wrote again: the
+// filter stage of one 640x480 frame went from 72 to 60 us, of the 64-session
+// step (frames read from pinned memory) from 1.12 to 0.98 ms.
 // ---------------------------------------------------------------------------
 __device__ inline int level_of_tile(const SessionDev& s, int tile_w, int tile_h, int& t) {
   int l = 0;
@@ -198,50 +211,57 @@ __device__ inline bool bp_valid(const float* depth, int w, int x, int y, const f
   return true;
 }
 
+constexpr int kMapRows = 32;  // a tile of the map passes is 32 x kMapRows pixels, 8 rows at a time
+
 __global__ void __launch_bounds__(256) k_inmap_pre(const BatchTable* __restrict__ bt) {
   const int n = bt->n;
-  const int total = bt->ipre[n];
+  const int total = bt->imap[n];
   for (int item = blockIdx.x; item < total; item += gridDim.x) {
     int t;
-    const int slot = find_slot(bt->ipre, n, item, t);
+    const int slot = find_slot(bt->imap, n, item, t);
     const SessionDev& s = *bt->s[slot];
-    const int l = level_of_tile(s, 32, 8, t);
+    const int l = level_of_tile(s, 32, kMapRows, t);
     const int w = s.lv[l].W, h = s.lv[l].H;
     const float K[4] = {s.lv[l].K[0], s.lv[l].K[1], s.lv[l].K[2], s.lv[l].K[3]};
     const float* __restrict__ depth = s.depth[l];
-    const int tw = (w + 31) / 32;
-    const int x = (t % tw) * 32 + threadIdx.x, y = (t / tw) * 8 + threadIdx.y;
-    if (y >= h) continue;  // whole warp (a warp is one 32-pixel row segment)
-    uint8_t code = 0;
-    float4 nv = make_float4(-100.0f, -100.0f, -100.0f, 0.0f);
-    if (x >= 1 && x < w - 1 && y >= 1 && y < h - 1) {
-      F3 c, x1, x2, y1, y2;
-      bool ok = bp_valid(depth, w, x, y, K, c) && bp_valid(depth, w, x - 1, y, K, x1) &&
-                bp_valid(depth, w, x + 1, y, K, x2) && bp_valid(depth, w, x, y - 1, K, y1) &&
-                bp_valid(depth, w, x, y + 1, K, y2);
-      if (ok) {
-        float dx = x2.x - x1.x;
-        float dy = y2.y - y1.y;
-        if (!(fabsf(dx) < 1.0e-7f) && !(fabsf(dy) < 1.0e-7f)) {
-          float dzdx = (x2.z - x1.z) / dx;
-          float dzdy = (y2.z - y1.z) / dy;
-          float len = sqrtf(dzdx * dzdx + dzdy * dzdy + 1.0f);
-          float nx = dzdx / len, ny = dzdy / len, nz = -1.0f / len;
-          // -n_z < cos(60 deg), the threshold taken in double as the reference's cos()
-          if (-(double)nz < 0.50000000000000011) {
-            code = 2;
-          } else {
-            code = 1;
-            nv = make_float4(nx, ny, nz, 0.0f);
+    const int tw = (w + 31) / 32, ty = t / tw, tx = t - ty * tw;
+    const int x = tx * 32 + threadIdx.x;
+#pragma unroll 1
+    for (int y = ty * kMapRows + threadIdx.y; y < min(h, (ty + 1) * kMapRows); y += 8) {
+      // a warp is one 32-pixel word of a row
+      int code = 0;
+      float4 nv = make_float4(-100.0f, -100.0f, -100.0f, 0.0f);
+      if (x >= 1 && x < w - 1 && y >= 1 && y < h - 1) {
+        F3 c, x1, x2, y1, y2;
+        bool ok = bp_valid(depth, w, x, y, K, c) && bp_valid(depth, w, x - 1, y, K, x1) &&
+                  bp_valid(depth, w, x + 1, y, K, x2) && bp_valid(depth, w, x, y - 1, K, y1) &&
+                  bp_valid(depth, w, x, y + 1, K, y2);
+        if (ok) {
+          float dx = x2.x - x1.x;
+          float dy = y2.y - y1.y;
+          if (!(fabsf(dx) < 1.0e-7f) && !(fabsf(dy) < 1.0e-7f)) {
+            float dzdx = (x2.z - x1.z) / dx;
+            float dzdy = (y2.z - y1.z) / dy;
+            float len = sqrtf(dzdx * dzdx + dzdy * dzdy + 1.0f);
+            float nz = -1.0f / len;
+            // -n_z < cos(60 deg), the threshold taken in double as the reference's cos():
+            // a float is below it iff it is at most 0.5
+            if (-nz <= 0.5f) {
+              code = 2;
+            } else {
+              code = 1;
+              nv = make_float4(dzdx / len, dzdy / len, nz, 1.0f);
+            }
           }
         }
       }
+      const unsigned m2 = __ballot_sync(0xffffffffu, code == 2), m1 = __ballot_sync(0xffffffffu, code == 1);
+      if (threadIdx.x == 0) {
+        s.in_amask[l][y * tw + tx] = m2;
+        s.in_cmask[l][y * tw + tx] = m1;
+      }
+      if (x < w) s.in_nrm[l][(size_t)y * w + x] = nv;
     }
-    const unsigned m = __ballot_sync(0xffffffffu, code == 2);
-    if (threadIdx.x == 0) s.in_amask[l][(size_t)y * tw + (t % tw)] = m;
-    if (x >= w) continue;
-    s.in_code[l][(size_t)y * w + x] = code;
-    s.in_nrm[l][(size_t)y * w + x] = nv;
   }
 }
 
@@ -249,41 +269,44 @@ __global__ void __launch_bounds__(256) k_inmap_pre(const BatchTable* __restrict_
 // lane l solves row t - l for its words, taking the carry of the row's earlier
 // words from lane l - 1 (computed at step t - 1) and the rejections of the row
 // above from its own registers, so one step costs one shuffle.  am: the
-// level's code-2 bitmasks (shared memory when they fit, else global).
-__device__ void scan_level(const uint32_t* am, uint32_t* __restrict__ rmask, int w, int h) {
+// level's code-2 bitmasks; rm receives the rejections (the same array where
+// they are in shared memory: a word is read one step before it is written).
+__device__ __forceinline__ void scan_level(const uint32_t* am, uint32_t* rm, int w, int h) {
   const int nw = (w + 31) >> 5;
   const int lane = threadIdx.x & 31;
   const uint32_t M0 = 0x55555555u, M1 = 0xaaaaaaaau;
   const int wpl = (nw + 31) >> 5;  // words per lane (1 up to 1024 pixels, 2 up to 2048)
   const int steps = h + 31;
   if (wpl == 1) {
-    // both outcomes of a word are formed before its carry arrives, so a step's
-    // critical path is one shuffle and one select
+    // Both outcomes of a word are formed before its carry arrives (a carry
+    // travels as a mask of 32 equal bits, so that choosing is one logic
+    // operation), the next word is read a step ahead, and rows outside the
+    // image hold no code, so they need no test: a step's critical path is a
+    // chain of eight operations from the row above, beside one of a shuffle
+    // and four.  Row 0 is never processed (interior rows only).
     const bool act = lane < nw;
-    uint32_t rup = 0u, cout = 0u;
-    for (int t = 0; t < steps; t++) {
-      const int row = t - lane;
-      const bool valid = act && row >= 0 && row < h;
-      uint32_t R0 = 0u, R1 = 0u;
-      if (valid && row > 0) {  // row 0 is never processed (interior rows only)
-        const uint32_t C = am[row * nw + lane] & ~rup;
-        const uint32_t st = C & ~(C << 1);  // run starts (bit 0 counted as a start)
-        const uint32_t ev = (C & ((C + ((st & ~1u) & M0)) ^ C)) & M0;
-        const uint32_t od = (C & ((C + ((st & ~1u) & M1)) ^ C)) & M1;
-        // a run at bit 0 continues the previous word's alternation: even
-        // parity after a clear carry, odd after a set one
-        const uint32_t b0 = st & 1u;
-        R0 = ev | ((C & ((C + b0) ^ C)) & M0) | od;
-        R1 = ev | od | ((C & ((C + b0) ^ C)) & M1);
-      }
-      uint32_t cin = __shfl_up_sync(0xffffffffu, cout, 1);
-      if (lane == 0) cin = 0u;
-      const uint32_t R = cin ? R1 : R0;
-      if (valid) {
-        rmask[(size_t)row * nw + lane] = R;
-        rup = R;
-      }
-      cout = valid ? (R >> 31) : 0u;
+    const uint32_t not_first = lane ? ~0u : 0u;
+    const unsigned rows = act ? (unsigned)h : 0u, ahead = act ? (unsigned)h - 1u : 0u;  // none for an idle lane
+    uint32_t rup = 0u, cout = 0u, next = 0u, next1 = 0u;
+    int i = lane - lane * nw;  // word of row t - lane
+#pragma unroll 4
+    for (int t = 0; t < steps; t++, i += nw) {
+      const unsigned row = (unsigned)(t - lane);
+      const uint32_t C = next & ~rup, C1 = next1 & ~(rup << 1);  // C1 = C << 1
+      next = 0u;
+      if (row < ahead) next = am[i + nw];
+      next1 = next << 1;
+      // run starts at even and odd bits (C & ~C1; one at bit 0 apart), and the
+      // runs they smear over
+      const uint32_t e = C + (C & ~C1 & (M0 & ~1u)), o = C + (C & ~C1 & M1), z = C + (C & 1u);
+      const uint32_t both = C & (((e ^ C) & M0) | ((o ^ C) & M1)), zero = C & (z ^ C);
+      // a run at bit 0 continues the previous word's alternation: even
+      // parity after a clear carry, odd after a set one
+      const uint32_t cin = __shfl_up_sync(0xffffffffu, cout, 1) & not_first;
+      const uint32_t R = both | (zero & (M0 ^ cin));
+      if (row < rows) rm[i] = R;
+      rup = R;
+      cout = (uint32_t)((int)R >> 31);
     }
     return;
   }
@@ -308,7 +331,7 @@ __device__ void scan_level(const uint32_t* am, uint32_t* __restrict__ rmask, int
             const uint32_t so = (rest & M1) | (cin ? (st & 1u) : 0u);
             R = ((C & ((C + se) ^ C)) & M0) | ((C & ((C + so) ^ C)) & M1);
           }
-          rmask[(size_t)row * nw + wi] = R;
+          rm[row * nw + wi] = R;
           rup[q] = R;
           cin = R >> 31;
         }
@@ -319,61 +342,153 @@ __device__ void scan_level(const uint32_t* am, uint32_t* __restrict__ rmask, int
   }
 }
 
+// i / n for 0 <= i < 2^14 and 1 <= n <= 64 without an integer division: (i +
+// 0.5) / n lies at least 0.5 / n from every integer, far more than the float
+// rounding of (i + 0.5) * (1 / n)
+__device__ __forceinline__ int small_div(int i, float inv_n) { return (int)(((float)i + 0.5f) * inv_n); }
+
+// the valid normals of word i (row y, word k of nw) from the code-1 mask and
+// the rejections
+__device__ __forceinline__ uint32_t valid_word(uint32_t code1, const uint32_t* rm, int i, int y, int k, int nw) {
+  const uint32_t left = (rm[i] << 1) | (k > 0 ? rm[i - 1] >> 31 : 0u), up = y > 0 ? rm[i - nw] : 0u;
+  return code1 & ~left & ~up;
+}
+
 // one block per (session, level) item
 __global__ void __launch_bounds__(1024) k_inmap_scan(const BatchTable* __restrict__ bt) {
-  extern __shared__ uint32_t amask[];  // [h][nw] of the current item
+  extern __shared__ uint32_t mask[];  // [h][nw] of the current item: code 2, then rejections
+  __shared__ int wsum[33];
   const int n = bt->n;
   const int total = bt->scan[n];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int item = blockIdx.x; item < total; item += gridDim.x) {
     int l;
     const int slot = find_slot(bt->scan, n, item, l);
     const SessionDev& s = *bt->s[slot];
     const int w = s.lv[l].W, h = s.lv[l].H;
-    const int nwords = h * ((w + 31) >> 5);
-    const uint32_t* src = s.in_amask[l];
+    const int nw = (w + 31) >> 5, nwords = h * nw;
+    const uint32_t* __restrict__ src = s.in_amask[l];
+    const uint32_t* __restrict__ cm = s.in_cmask[l];
+    uint32_t* rm = s.in_rmask[l];
+    // the valid normals before each word are counted by all warps: each takes
+    // `strips` runs of 32 words, and reads its code-1 words before the sweep
+    constexpr int kStrips = kScanSmem / 4 / 1024;
+    const int strips = (nwords + 1023) / 1024;
+    const int first = warp * strips * 32 + lane;
     const bool staged = nwords * 4 <= kScanSmem;
-    if (staged)
-      for (int i = threadIdx.x; i < nwords; i += blockDim.x) amask[i] = src[i];
+    uint32_t c1[kStrips];
+    if (staged) {
+      for (int i = threadIdx.x; i < nwords; i += blockDim.x) mask[i] = src[i];
+#pragma unroll
+      for (int q = 0; q < kStrips; q++) c1[q] = (q < strips && first + q * 32 < nwords) ? cm[first + q * 32] : 0u;
+    }
     __syncthreads();
-    if (threadIdx.x < 32) scan_level(staged ? amask : src, s.in_rmask[l], w, h);
+    if (warp == 0) {
+      if (staged)
+        scan_level(mask, mask, w, h);
+      else
+        scan_level(src, rm, w, h);
+    }
+    __syncthreads();
+    const float inv = 1.0f / (float)nw;
+    int sum = 0;  // the lane's words
+    if (staged) {
+#pragma unroll
+      for (int q = 0; q < kStrips; q++) {
+        const int i = first + q * 32;
+        if (q < strips && i < nwords) {
+          const int y = small_div(i, inv);
+          c1[q] = (uint32_t)__popc(valid_word(c1[q], mask, i, y, i - y * nw, nw));
+          sum += (int)c1[q];
+          rm[i] = mask[i];
+        }
+      }
+    } else {
+      for (int q = 0; q < strips; q++) {
+        const int i = first + q * 32;
+        if (i < nwords) {
+          const int y = i / nw;
+          sum += __popc(valid_word(cm[i], rm, i, y, i - y * nw, nw));
+        }
+      }
+    }
+    sum = __reduce_add_sync(0xffffffffu, sum);
+    if (lane == 0) wsum[warp] = sum;
+    __syncthreads();
+    int base = 0;  // before the warp's words
+    {
+      const int v = wsum[lane];
+      base = __reduce_add_sync(0xffffffffu, lane < warp ? v : 0);
+      const int all = __reduce_add_sync(0xffffffffu, v);
+      if (threadIdx.x == 0) s.in_count[l] = (uint32_t)all;
+    }
+    auto prefix = [&](int i, int c) {
+      int v = c;
+#pragma unroll
+      for (int m = 1; m < 32; m <<= 1) {
+        const int o = __shfl_up_sync(0xffffffffu, v, m);
+        if (lane >= m) v += o;
+      }
+      if (i < nwords) s.in_base[l][i] = (uint32_t)(base + v - c);
+      base += __shfl_sync(0xffffffffu, v, 31);
+    };
+    if (staged) {
+#pragma unroll
+      for (int q = 0; q < kStrips; q++)
+        if (q < strips) prefix(first + q * 32, (int)c1[q]);
+    } else {
+      for (int q = 0; q < strips; q++) {
+        const int i = first + q * 32;
+        int c = 0;
+        if (i < nwords) {
+          const int y = i / nw;
+          c = __popc(valid_word(cm[i], rm, i, y, i - y * nw, nw));
+        }
+        prefix(i, c);
+      }
+    }
     __syncthreads();  // the next item restages the shared masks
   }
 }
 
 __global__ void __launch_bounds__(256) k_inmap_post(const BatchTable* __restrict__ bt) {
   const int n = bt->n;
-  const int total = bt->ipost[n];
+  const int total = bt->imap[n];
   for (int item = blockIdx.x; item < total; item += gridDim.x) {
     int t;
-    const int slot = find_slot(bt->ipost, n, item, t);
+    const int slot = find_slot(bt->imap, n, item, t);
     const SessionDev& s = *bt->s[slot];
-    const int l = level_of_tile(s, 16, 16, t);
+    const int l = level_of_tile(s, 32, kMapRows, t);
     const int w = s.lv[l].W, h = s.lv[l].H;
-    const int tw = (w + 15) / 16;
-    const int x = (t % tw) * 16 + threadIdx.x, y = (t / tw) * 16 + threadIdx.y;
-    if (x >= w || y >= h) continue;
-    const int nw = (w + 31) >> 5;
+    const int nw = (w + 31) >> 5, ty = t / nw, k = t - ty * nw;
+    const int x = k * 32 + threadIdx.x;
+    if (x >= w) continue;
+    const float K[4] = {s.lv[l].K[0], s.lv[l].K[1], s.lv[l].K[2], s.lv[l].K[3]};
     const uint32_t* __restrict__ rm = s.in_rmask[l];
-    auto rej = [&](int xx, int yy) -> bool {
-      if (xx < 0 || yy < 0) return false;
-      return (rm[(size_t)yy * nw + (xx >> 5)] >> (xx & 31)) & 1u;
-    };
-    const size_t idx = (size_t)y * w + x;
-    const float d = s.depth[l][idx];
-    float4 v = make_float4(-100.0f, -100.0f, -100.0f, 0.0f);
-    if (d > 0.0f && !rej(x, y)) {
-      F3 p = back_project((float)x, (float)y, s.lv[l].K, d);
-      v = make_float4(p.x, p.y, p.z, 1.0f);
+    const uint32_t* __restrict__ cm = s.in_cmask[l];
+    const uint32_t* __restrict__ base = s.in_base[l];
+    const float* __restrict__ depth = s.depth[l];
+    float4* __restrict__ vtx = s.in_vtx[l];
+    float4* __restrict__ nrm = s.in_nrm[l];
+    uint32_t* __restrict__ list = s.in_list[l];
+    const uint32_t bit = 1u << threadIdx.x;
+#pragma unroll 2
+    for (int y = ty * kMapRows + threadIdx.y; y < min(h, (ty + 1) * kMapRows); y += 8) {
+      // a warp is one 32-pixel word of a row
+      const int i = y * nw + k;
+      const uint32_t code1 = cm[i];
+      const uint32_t valid = valid_word(code1, rm, i, y, k, nw);
+      const size_t idx = (size_t)y * w + x;
+      const float d = depth[idx];
+      float4 v = make_float4(-100.0f, -100.0f, -100.0f, 0.0f);
+      if (d > 0.0f && !(rm[i] & bit)) {
+        F3 p = back_project((float)x, (float)y, K, d);
+        v = make_float4(p.x, p.y, p.z, 1.0f);
+      }
+      vtx[idx] = v;
+      if (code1 & ~valid & bit) nrm[idx] = make_float4(-100.0f, -100.0f, -100.0f, 0.0f);
+      if (valid & bit) list[base[i] + __popc(valid & (bit - 1u))] = (uint32_t)((y << 16) | x);
     }
-    s.in_vtx[l][idx] = v;
-    const uint8_t code = s.in_code[l][idx];
-    float4 nv = s.in_nrm[l][idx];
-    if (code == 1 && !rej(x - 1, y) && !rej(x, y - 1)) {
-      nv.w = 1.0f;
-    } else {
-      nv = make_float4(-100.0f, -100.0f, -100.0f, 0.0f);
-    }
-    s.in_nrm[l][idx] = nv;
   }
 }
 
@@ -399,7 +514,7 @@ void launch_input_maps(const BatchTable* bt, cudaStream_t st) {
   const int grid = sm_count() * 8;
   k_inmap_pre<<<grid, dim3(32, 8), 0, st>>>(bt);
   k_inmap_scan<<<kMaxSlots * kMaxLevels, 1024, kScanSmem, st>>>(bt);
-  k_inmap_post<<<grid, dim3(16, 16), 0, st>>>(bt);
+  k_inmap_post<<<grid, dim3(32, 8), 0, st>>>(bt);
 }
 
 void launch_bilateral_float(const SessionDev& h, const float* in, float* out, cudaStream_t st) {
@@ -425,19 +540,17 @@ void fill_batch_table(BatchTable& hb, const SessionDev* const* host_recs, const 
     const SessionDev& h = *host_recs[i];
     hb.s[i] = dev_recs[i];
     const bool nm = h.cos_normal > -2.0f;
-    int ipre = 0, ipost = 0, ray = 0;
+    int imap = 0, ray = 0;
     for (int l = 0; l < h.levels; l++) {
       const int w = h.lv[l].W, hh = h.lv[l].H;
-      ipre += ((w + 31) / 32) * ((hh + 7) / 8);
-      ipost += ((w + 15) / 16) * ((hh + 15) / 16);
+      imap += ((w + 31) / 32) * ((hh + kMapRows - 1) / kMapRows);
       ray += ((w + rx - 1) / rx) * ((hh + ry - 1) / ry);
     }
     hb.bil[i + 1] = hb.bil[i] + ((h.lv[0].W + BX - 1) / BX) * ((h.lv[0].H + hb.bil_rows - 1) / hb.bil_rows);
     for (int l = 1; l < kMaxLevels; l++)
       hb.pyr[l - 1][i + 1] =
           hb.pyr[l - 1][i] + (l < h.levels ? ((h.lv[l].W + 31) / 32) * ((h.lv[l].H + 7) / 8) : 0);
-    hb.ipre[i + 1] = hb.ipre[i] + (nm ? ipre : 0);
-    hb.ipost[i + 1] = hb.ipost[i] + (nm ? ipost : 0);
+    hb.imap[i + 1] = hb.imap[i] + (nm ? imap : 0);
     hb.scan[i + 1] = hb.scan[i] + (nm ? h.levels : 0);
     for (int l = 0; l < kMaxLevels; l++)
       hb.icp[l][i + 1] = hb.icp[l][i] + (l < h.levels ? icp_blocks(h.lv[l].W * h.lv[l].H, l) : 0);

@@ -773,6 +773,24 @@ __device__ __noinline__ void claim_range(unsigned* __restrict__ words, int n, co
   }
 }
 
+// Ranges of a level whose pixels are listed: a session that tests normals has
+// no term where the input normal is invalid, so its ranges run over the list
+// of the pixels with a valid one (in raster order).  Those are 5 to 15 % of
+// the pixels of the serving mix (the 60 degree test of the normal estimation
+// on noisy depth), in 15 to 30 % of the 32-pixel words.  Reading depth and model
+// taps of every pixel, tracking took 2.01 ms of the 64-session step and 0.606
+// of sixteen sessions'; over the list 0.52 and 0.26 (a 640x480 frame 490 ->
+// 434 us).  512 pixels per range: 256 and 1024 made a 640x480 frame 422 and 462
+// us, the 64-session step 4712 and 4456 us against 4505.  Every session has
+// at least one range, which closes its iterations.
+#ifndef VS_ICP_LISTED_PER_RANGE
+#define VS_ICP_LISTED_PER_RANGE 512
+#endif
+__device__ __forceinline__ int listed_ranges(int count) {
+  const int r = (count + VS_ICP_LISTED_PER_RANGE - 1) / VS_ICP_LISTED_PER_RANGE;
+  return min(max(r, 1), kIcpMaxBlocks);
+}
+
 // a load that the compiler does not merge with an earlier one
 template <class T>
 __device__ __forceinline__ T reload(const T* p) {
@@ -794,8 +812,13 @@ __global__ void __launch_bounds__(kThreads, VS_ICP_MIN_BLOCKS)
   if (threadIdx.x < kMaxSlots) {
     const int i = threadIdx.x;
     sS[i] = i < n ? bt->s[i] : nullptr;
+    const bool listed = i < n && sS[i]->cos_normal > -2.0f;
 #pragma unroll
-    for (int l = 0; l < kMaxLevels; l++) sNvb[l][i] = i < n ? bt->icp[l][i + 1] - bt->icp[l][i] : 0;
+    for (int l = 0; l < kMaxLevels; l++) {
+      int r = i < n ? bt->icp[l][i + 1] - bt->icp[l][i] : 0;
+      if (r && listed) r = listed_ranges((int)sS[i]->in_count[l]);
+      sNvb[l][i] = r;
+    }
     sNvb[kMaxLevels][i] = 0;
   }
   __syncthreads();
@@ -823,32 +846,49 @@ __global__ void __launch_bounds__(kThreads, VS_ICP_MIN_BLOCKS)
 
     Acc<MODE> acc;
     acc.zero();
-    const int npix = w * h;
-    const int stride = nvb * kThreads;
     const bool ntest = cosn > -2.0f;
+    const uint32_t* list = ntest ? s->in_list[level] : nullptr;
+    const int count = ntest ? (int)s->in_count[level] : w * h;
+    const int stride = nvb * kThreads;
     // the first-round reads (depth, input normal) of a thread's next pixel are
-    // in flight while its current pixel's taps are read
+    // in flight while its current pixel's taps are read, and the list entry
+    // of the one after that
     int p = vb * kThreads + threadIdx.x;
-    int y = p / w, x = p - y * w;
-    const int dy = stride / w, dx = stride - dy * w;
+    int x = 0, y = 0, dx = 0, dy = 0;
+    uint32_t xy = 0u;
     float d_next = 0.0f;
     float4 q_next = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    if (p < npix) {
-      d_next = __ldg(depth + p);
-      if (ntest) q_next = __ldg(innrm + p);
+    if (ntest) {
+      if (p < count) {
+        xy = __ldg(list + p);
+        x = (int)(xy & 0xffffu), y = (int)(xy >> 16);
+        d_next = __ldg(depth + y * w + x);
+        q_next = __ldg(innrm + y * w + x);
+        if (p + stride < count) xy = __ldg(list + p + stride);
+      }
+    } else {
+      y = p / w, x = p - y * w;
+      dy = stride / w, dx = stride - dy * w;
+      if (p < count) d_next = __ldg(depth + p);
     }
     __syncthreads();
-    while (p < npix) {
+    while (p < count) {
       const float d1 = d_next;
       const float4 qn = q_next;
       const int xc = x, yc = y;
       p += stride;
-      x += dx;
-      y += dy;
-      if (x >= w) x -= w, y++;
-      if (p < npix) {
-        d_next = __ldg(depth + p);
-        if (ntest) q_next = __ldg(innrm + p);
+      if (ntest) {
+        if (p < count) {
+          x = (int)(xy & 0xffffu), y = (int)(xy >> 16);
+          d_next = __ldg(depth + y * w + x);
+          q_next = __ldg(innrm + y * w + x);
+          if (p + stride < count) xy = __ldg(list + p + stride);
+        }
+      } else {
+        x += dx;
+        y += dy;
+        if (x >= w) x -= w, y++;
+        if (p < count) d_next = __ldg(depth + p);
       }
       float A[6], b;
       if (!icp_term(xc, yc, w, h, K, d1, qn, mvtx, mnrm, T21, th, cosn, A, b)) continue;

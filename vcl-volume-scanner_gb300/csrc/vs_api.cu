@@ -159,6 +159,7 @@ int reset_state(vs_session* s) {
   launch_occupancy_clear(s->h, s->stream);
   VS_CU(cudaGetLastError());
   VS_CU(cudaMemsetAsync(s->h.icp_counter, 0, sizeof(unsigned), s->stream));
+  VS_CU(cudaMemsetAsync(s->h.in_count, 0, kMaxLevels * sizeof(uint32_t), s->stream));
   Pose p;
   std::memset(&p, 0, sizeof(p));
   for (int i = 0; i < 16; i++) {
@@ -281,8 +282,9 @@ size_t vs_session_bytes(const vs_config* c) {
   b += (size_t)w * h * (2 + 4 + 4);
   for (int l = 0; l < c->levels; l++) {
     size_t n = (size_t)(w >> l) * (h >> l);
-    b += n * (4 + 16 + 16 + 1 + 4 + 16 + 16 + 1) + 2 * (size_t)(h >> l) * (((w >> l) + 31) / 32) * 4;
+    b += n * (4 + 16 + 16 + 4 + 4 + 16 + 16 + 1) + 4 * (size_t)(h >> l) * (((w >> l) + 31) / 32) * 4;
   }
+  b += 64;  // valid-normal counts
   b += (size_t)kIcpMaxBlocks * kPartials * 16 + sizeof(Pose) + sizeof(SessionDev) + sizeof(BatchTable) + 64;
   b += (size_t)(c->dim[0] + c->dim[1] + c->dim[2] + w + h) * 4;
   for (int l = 0; l < c->levels; l++) b += (size_t)(w >> l) * (h >> l) * 16;  // ray-cast hit points
@@ -340,9 +342,12 @@ int vs_session_create(const vs_config* cfg, vs_session** out) {
     rc |= alloc(s, &h.depth[l], n * 4);
     rc |= alloc(s, &h.in_vtx[l], n * 16);
     rc |= alloc(s, &h.in_nrm[l], n * 16);
-    rc |= alloc(s, &h.in_code[l], n);
-    rc |= alloc(s, &h.in_amask[l], (size_t)h.lv[l].H * ((h.lv[l].W + 31) / 32) * 4);
-    rc |= alloc(s, &h.in_rmask[l], (size_t)h.lv[l].H * ((h.lv[l].W + 31) / 32) * 4);
+    const size_t words = (size_t)h.lv[l].H * ((h.lv[l].W + 31) / 32);
+    rc |= alloc(s, &h.in_amask[l], words * 4);
+    rc |= alloc(s, &h.in_cmask[l], words * 4);
+    rc |= alloc(s, &h.in_rmask[l], words * 4);
+    rc |= alloc(s, &h.in_base[l], words * 4);
+    rc |= alloc(s, &h.in_list[l], n * 4);
     rc |= alloc(s, &h.m_depth[l], n * 4);
     rc |= alloc(s, &h.m_vtx[l], n * 16);
     rc |= alloc(s, &h.m_nrm[l], n * 16);
@@ -350,6 +355,7 @@ int vs_session_create(const vs_config* cfg, vs_session** out) {
   }
   rc |= alloc(s, &h.partials, (size_t)kIcpMaxBlocks * kPartials * 16);
   rc |= alloc(s, &h.icp_counter, 64);
+  rc |= alloc(s, &h.in_count, 64);
   rc |= alloc(s, &h.pose, sizeof(Pose));
   rc |= alloc(s, &h.lut_vox, (size_t)(h.dim[0] + h.dim[1] + h.dim[2]) * 4);
   rc |= alloc(s, &h.lut_ray, (size_t)(h.lv[0].W + h.lv[0].H) * 4);

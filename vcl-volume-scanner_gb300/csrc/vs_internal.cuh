@@ -68,9 +68,12 @@ struct SessionDev {
   float* depth[kMaxLevels];      // filtered pyramid
   float4* in_vtx[kMaxLevels];    // input vertex map (w = 1 valid, 0 invalid)
   float4* in_nrm[kMaxLevels];    // input normal map (w = 1 valid)
-  uint8_t* in_code[kMaxLevels];  // normal-map pre-pass codes
   uint32_t* in_amask[kMaxLevels];// per-row bitmasks of normals failing the angle test
-  uint32_t* in_rmask[kMaxLevels];// per-row rejection bitmasks
+  uint32_t* in_cmask[kMaxLevels];// of normals passing it
+  uint32_t* in_rmask[kMaxLevels];// rejection bitmasks
+  uint32_t* in_base[kMaxLevels]; // valid normals before each word of the masks
+  uint32_t* in_list[kMaxLevels]; // the pixels with a valid normal in raster order, y << 16 | x
+  uint32_t* in_count;            // their number per level
   float* m_depth[kMaxLevels];    // model (ray-cast) maps
   float4* m_vtx[kMaxLevels];     // xyz, w = 1 valid (invalid: -100)
   float4* m_nrm[kMaxLevels];
@@ -119,8 +122,7 @@ struct BatchTable {
   const SessionDev* s[kMaxSlots];
   int bil[kMaxSlots + 1];              // level-0 32 x bil_rows tiles (bilateral, activation)
   int pyr[kMaxLevels - 1][kMaxSlots + 1];  // 32x8 tiles of levels 1, 2
-  int ipre[kMaxSlots + 1];             // input-map pre-pass 32x8 tiles, all levels
-  int ipost[kMaxSlots + 1];            // input-map post-pass 16x16 tiles, all levels
+  int imap[kMaxSlots + 1];             // input-map 32x32 tiles, all levels
   int scan[kMaxSlots + 1];             // input-map row scans: one per level
   int icp[kMaxLevels][kMaxSlots + 1];  // ICP block ranges per level
   int ray[kMaxSlots + 1];              // ray-cast tiles, all levels
