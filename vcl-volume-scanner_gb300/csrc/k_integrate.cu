@@ -315,14 +315,6 @@ __device__ void color_round(const IP& q, unsigned upd, int v0, int lane, int bx,
 #define VS_INT_MIN_BLOCKS 4  // resident 256-thread blocks per SM the register allocation must allow
 #endif
 
-// rcp.approx.ftz.f32: the reciprocal with at most 1 ulp of error (PTX ISA,
-// "rcp.approx"), one special-function instruction
-__device__ __forceinline__ float rcp_approx(float z) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(z));
-  return r;
-}
-
 // Nearest pixel of a camera-frame point: (__float2int_rn(u), __float2int_rn(v))
 // of d_p_Project's u = K0 x / z + K2, v = K1 y / z + K3 with IEEE division
 // (_yooji_cuda_math.h:205-210, z_yooji_cuda_volume_integrator.cu:344-347),

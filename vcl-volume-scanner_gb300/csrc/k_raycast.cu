@@ -58,7 +58,7 @@ template <class S>
 struct Vol {
   const typename S::word* v;
   const uint8_t* bdist;  // distance in bricks to the nearest band brick
-  int dim[3];
+  float dim[3];
   uint32_t nbx, nbxy;  // bricks per row / per slab
   uint32_t sy, sz;  // word strides of one brick row / one brick slab: 512 nb[0], 512 nb[0] nb[1]
   // The word index of voxel (x, y, z) >= 0 is the sum of one term per axis
@@ -70,9 +70,33 @@ struct Vol {
   __device__ inline uint32_t wz(int z) const { return ((uint32_t)z >> 3) * sz + (((uint32_t)z & 7u) << 6); }
   // the value of word i, and whether its weight is > 0
   __device__ inline bool word_ok(uint32_t i, float& t) const {
-    uint32_t w;
-    S::decode(__ldg(v + i), t, w);
-    return w != 0u;
+    const typename S::word u = __ldg(v + i);
+    t = S::value(u);
+    return S::weighted(u);
+  }
+  // The nearest voxel of p (ROUNDF), and whether it is in range.  ROUNDF(p) is
+  // negative for every p <= -0.5 and equals (int)(p + 0.5) for every p > -0.5
+  // (both branches give 0 on (-0.5, 0)), so one comparison per coordinate
+  // decides the lower bound, and a NaN coordinate fails it too; the integer
+  // part of p + 0.5 is below dim iff p + 0.5 is.
+  struct Near {
+    int x, y, z;
+    bool in;
+  };
+  __device__ inline Near nearest(F3 p) const {
+    const float x = p.x + 0.5f, y = p.y + 0.5f, z = p.z + 0.5f;
+    Near v;
+    v.in = p.x > -0.5f && p.y > -0.5f && p.z > -0.5f && x < dim[0] && y < dim[1] && z < dim[2];
+    v.x = (int)x, v.y = (int)y, v.z = (int)z;
+    return v;
+  }
+  // d_gtvu_Get_TSDF_Value_Uninterpolated: nearest voxel, weight > 0
+  __device__ inline bool gtvu(const Near& v, float& out) const {
+    out = 1.0f;
+    float t;
+    if (!v.in || !word_ok(wx(v.x) + wy(v.y) + wz(v.z), t)) return false;
+    out = t;
+    return true;
   }
   // Free-space run: how many of the next steps p + k inc (k = 1..m) are
   // certain to read TSDF 1 ("no value", or a voxel whose value is 1) -
@@ -91,29 +115,27 @@ struct Vol {
   // and gives 0.
   static constexpr int kMaxRun = 4096;
   static constexpr int kMaxBoxes = 2;
-  __device__ inline int free_run(F3 p, F3 inc) const {
+  __device__ inline int free_run(F3 p, F3 inc, const Near& near) const {
     const float d = 0.05f;
     const float pa[3] = {p.x, p.y, p.z}, ia[3] = {inc.x, inc.y, inc.z};
-    const float ra[3] = {__fdividef(1.0f, inc.x), __fdividef(1.0f, inc.y), __fdividef(1.0f, inc.z)};
+    const float ra[3] = {rcp_approx(inc.x), rcp_approx(inc.y), rcp_approx(inc.z)};
     int run = 0;
+#pragma unroll
     for (int j = 0; j < kMaxBoxes; j++) {
       // q: step `run` (j = 0: the current sample, which read 1; after that
       // the step following the last box, a candidate for the run)
       float q[3];
 #pragma unroll
       for (int a = 0; a < 3; a++) q[a] = j == 0 ? pa[a] : (float)run * ia[a] + pa[a];
-      // a coordinate is in range iff -0.5 < q < dim - 0.5 (gtvu rounds with ROUNDF)
-      bool inside = true;
-#pragma unroll
-      for (int a = 0; a < 3; a++) inside &= q[a] > -0.5f && q[a] < (float)dim[a] - 0.5f;
+      const Near v = j == 0 ? near : nearest(f3(q[0], q[1], q[2]));
       float t;
       bool band = false, sure = false;  // sure: q reads 1 however it rounds
-      if (!inside) {
+      if (!v.in) {
         // outside until every coordinate that is out of range has come in
         t = 0.0f;
 #pragma unroll
         for (int a = 0; a < 3; a++) {
-          const float hi = (float)dim[a] - 0.5f;
+          const float hi = dim[a] - 0.5f;
           if (q[a] <= -0.5f) {
             t = fmaxf(t, ia[a] > 0.0f ? (-0.5f - d - q[a]) * ra[a] : 1e30f);
             sure |= q[a] < -0.5f - d;
@@ -123,66 +145,49 @@ struct Vol {
           }
         }
       } else {
-        // inside: every coordinate > -0.5, where ROUNDF is (int)(q + 0.5);
-        // brick b holds the nearest voxel, and the box of bricks b - h ..
-        // b + h (h = bdist - 1) holds no band brick; in a band brick (bdist
-        // 0) the box is the brick itself
-        const int b[3] = {(int)(q[0] + 0.5f) >> 3, (int)(q[1] + 0.5f) >> 3, (int)(q[2] + 0.5f) >> 3};
+        // brick b holds the nearest voxel, and the box of bricks b - h .. b + h
+        // (h = bdist - 1) holds no band brick; in a band brick (bdist
+        // 0) the box is the brick itself.  (The box bounds are halves, exact.)
+        const int b[3] = {v.x >> 3, v.y >> 3, v.z >> 3};
         const int dist = __ldg(bdist + (uint32_t)b[2] * nbxy + (uint32_t)b[1] * nbx + (uint32_t)b[0]);
         band = dist == 0;
         sure = !band;
-        const int h = band ? 0 : dist - 1;
+        const float h = band ? 0.0f : (float)(dist - 1), h1 = h + 1.0f;
         t = 1e30f;
 #pragma unroll
         for (int a = 0; a < 3; a++) {
-          const float lo = (float)((b[a] - h) * 8) - 0.5f, hi = (float)((b[a] + h + 1) * 8) - 0.5f;
-          sure &= q[a] > lo + d && q[a] < hi - d;
-          if (ia[a] > 0.0f)
-            t = fminf(t, (hi - d - q[a]) * ra[a]);
-          else if (ia[a] < 0.0f)
-            t = fminf(t, (lo + d - q[a]) * ra[a]);
+          const float bf = (float)b[a];
+          const float lo = fmaf(bf - h, 8.0f, -0.5f) + d, hi = fmaf(bf + h1, 8.0f, -0.5f) - d;
+          sure &= q[a] > lo && q[a] < hi;
+          const float u = ((ia[a] > 0.0f ? hi : lo) - q[a]) * ra[a];
+          if (ia[a] != 0.0f) t = fminf(t, u);
         }
       }
       if (j > 0 && !sure) return run - 1;
-      // steps k >= 1 from q with k < t
+      // steps k >= 1 from q with k < t: ceil(t) - 1
       t = fminf(t, (float)(kMaxRun + 1));
-      const int m = (int)ceilf(t) - 1;
-      if (j == 0 && band) return m > 0 ? -m : 0;
-      run += m > 0 ? m : 0;
+      const int m = max(__float2int_ru(t), 1) - 1;
+      if (j == 0 && band) return -m;
+      run += m;
       if (run >= kMaxRun) return run;
       run++;  // the next candidate
     }
     return run - 1;
   }
 
-  // d_gtvu_Get_TSDF_Value_Uninterpolated: nearest voxel (ROUNDF), weight > 0.
-  // ROUNDF(p) is negative for every p <= -0.5 and equals (int)(p + 0.5) for
-  // every p > -0.5 (both branches give 0 on (-0.5, 0)), so one comparison per
-  // coordinate decides the lower bound, and a NaN coordinate fails it too.
-  __device__ inline bool gtvu(F3 p, float& out) const {
-    out = 1.0f;
-    if (!(p.x > -0.5f && p.y > -0.5f && p.z > -0.5f)) return false;
-    const int x = (int)(p.x + 0.5f), y = (int)(p.y + 0.5f), z = (int)(p.z + 0.5f);
-    if (x >= dim[0] || y >= dim[1] || z >= dim[2]) return false;
-    const uint32_t i = wx(x) + wy(y) + wz(z);
-    float t;
-    if (!word_ok(i, t)) return false;
-    out = t;
-    return true;
-  }
   // d_gtvi_Get_TSDF_Value_Interpolated (offset = floor, see the oracle); the
   // eight reads have no side effects, so reading all of them before the
   // validity test gives the short-circuit form's result
   __device__ inline bool gtvi(F3 p, float& out) const {
     out = 1.0f;
-    if (isnan(p.x) || isnan(p.y) || isnan(p.z)) return false;
-    float fx = floorf(p.x), fy = floorf(p.y), fz = floorf(p.z);
-    int ox = (int)fx, oy = (int)fy, oz = (int)fz;
-    float rx = p.x - fx, ry = p.y - fy, rz = p.z - fz;
-    // the eight corners are in range iff both values of every axis are; an
-    // out-of-range value is clamped for its (discarded) read
-    bool ok = ox >= 0 && ox + 1 < dim[0] && oy >= 0 && oy + 1 < dim[1] && oz >= 0 && oz + 1 < dim[2];
-    const int cx = min(max(ox, 0), dim[0] - 2), cy = min(max(oy, 0), dim[1] - 2), cz = min(max(oz, 0), dim[2] - 2);
+    // the eight corners floor(p), floor(p) + 1 are in range iff 0 <= p < dim - 1
+    // (false for a NaN)
+    if (!(p.x >= 0.0f && p.x < dim[0] - 1.0f && p.y >= 0.0f && p.y < dim[1] - 1.0f && p.z >= 0.0f &&
+          p.z < dim[2] - 1.0f))
+      return false;
+    const int cx = (int)p.x, cy = (int)p.y, cz = (int)p.z;
+    const float rx = p.x - (float)cx, ry = p.y - (float)cy, rz = p.z - (float)cz;
+    bool ok = true;
     const uint32_t x0 = wx(cx), x1 = wx(cx + 1), y0 = wy(cy), y1 = wy(cy + 1), z0 = wz(cz), z1 = wz(cz + 1);
     float f0, f1, f2, f3_, b0, b1, b2, b3;
     ok &= word_ok(z0 + y0 + x0, f0);
@@ -207,19 +212,19 @@ template <class S>
 __device__ bool surface_normal(const Vol<S>& V, const SessionDev& s, F3 p3d, F3& nout) {
   F3 vox;
   if (!pos_in_voxel(p3d, s, vox)) return false;
-  if (isnan(vox.x) || isnan(vox.y) || isnan(vox.z)) return false;
-  float fx = floorf(vox.x), fy = floorf(vox.y), fz = floorf(vox.z);
-  const int ox = (int)fx, oy = (int)fy, oz = (int)fz;
-  const float rx = vox.x - fx, ry = vox.y - fy, rz = vox.z - fz;
+  // the stencil spans floor(v) - 1 .. floor(v) + 2 on every axis and uses each
+  // of those values, so it is in range iff 1 <= v < dim - 2 (false for a NaN)
+  if (!(vox.x >= 1.0f && vox.x < V.dim[0] - 2.0f && vox.y >= 1.0f && vox.y < V.dim[1] - 2.0f && vox.z >= 1.0f &&
+        vox.z < V.dim[2] - 2.0f))
+    return false;
+  const int cx = (int)vox.x, cy = (int)vox.y, cz = (int)vox.z;
+  const float rx = vox.x - (float)cx, ry = vox.y - (float)cy, rz = vox.z - (float)cz;
   const int dx1[4] = {0, 1, 0, 1}, dy1[4] = {0, 0, 1, 1};
   const int dx2[12] = {0, 1, -1, 0, 1, 2, -1, 0, 1, 2, 0, 1};
   const int dy2[12] = {-1, -1, 0, 0, 0, 0, 1, 1, 1, 1, 2, 2};
   // all 32 reads are issued before any validity test (no side effects, so
-  // the result equals the reference's read-and-return-early order).  The
-  // stencil spans o - 1 .. o + 2 on every axis and uses each of those values,
-  // so it is in range iff o - 1 >= 0 and o + 2 < dim on all three axes.
-  bool ok = ox >= 1 && ox + 2 < V.dim[0] && oy >= 1 && oy + 2 < V.dim[1] && oz >= 1 && oz + 2 < V.dim[2];
-  const int cx = min(max(ox, 1), V.dim[0] - 3), cy = min(max(oy, 1), V.dim[1] - 3), cz = min(max(oz, 1), V.dim[2] - 3);
+  // the result equals the reference's read-and-return-early order)
+  bool ok = true;
   uint32_t X[4], Y[4], Z[4];
 #pragma unroll
   for (int k = 0; k < 4; k++) X[k] = V.wx(cx - 1 + k), Y[k] = V.wy(cy - 1 + k), Z[k] = V.wz(cz - 1 + k);
@@ -281,56 +286,88 @@ __device__ bool surface_normal(const Vol<S>& V, const SessionDev& s, F3 p3d, F3&
   return true;
 }
 
-template <class S>
-__device__ bool cast_ray(const Vol<S>& V, const SessionDev& s, const float* K, float px, float py,
-                         const float* Tcg, F3 cam, float dmin, float dmax, bool cone, F3 ncc, float theta_max,
-                         F3& p3d) {
-  enum { COARSE, FINE, BEHIND };
-  F3 pe = transform(back_project(px, py, K, dmax), Tcg);
-  F3 rd = normalised(sub(pe, cam));
-  if (cone) {
-    float theta = acosf(dot(rd, ncc));
-    if (theta > theta_max) return false;
-  }
-  F3 ps = add(cam, scale(dmin, rd));
-  const float step_scale = 0.9f * s.mu * s.vox_inv;
-  const float total_max = 2.0f * s.r_cube * s.vox_inv;
-  float step, total = 0.0f, tsdf;
-  F3 vs;
-  pos_in_voxel(ps, s, vs);
+// What every ray of one level of one session has in common, in shared memory
+// per warp: formed when the warp's tiles come to another level or session
+// instead of by each lane for its ray (a tenth of a ray's instructions).
+struct TileCam {
+  float Tcg[12], Tgc[12];
+  F3 cam;             // camera centre
+  float theta_max;    // half angle of the cube's view cone
+  F3 ncc;             // direction of the cube's centre
+  float dmin, dmax;   // the marched segment
+  float K[4];
+  float step_scale, total_max;  // full step and length of the march, in voxels
+};
+
+// The state of a march
+struct March {
+  F3 vs;          // position in voxels
+  float total;    // distance marched
+  float tsdf;     // the sample there
   int state;
-  if (!V.gtvu(vs, tsdf))
-    state = COARSE;
-  else if (tsdf >= 0.0f)
-    state = FINE;
-  else
-    return false;
-  const int cap = 4 * (int)total_max + 64;
-  int it = 0;
-  int recheck = 0;  // full steps before the next free-space test
-  while (state != BEHIND) {
-    if (++it > cap) return false;
-    if (state == COARSE)
+  int recheck;    // full steps before the next free-space test
+};
+enum { COARSE, FINE, BEHIND };
+enum { kMarchMiss, kMarchZero, kMarchBehind, kMarchLong };
+
+__device__ __forceinline__ bool same_bits(float a, float b) { return __float_as_uint(a) == __float_as_uint(b); }
+// Whether two states take the same samples from here on: the next position,
+// sample and search state follow from these alone (a recheck of 0 or less is
+// due).  The distance and the iteration count differ, but all they can do is
+// end the march without a hit.
+__device__ __forceinline__ bool same_course(const March& a, const March& b) {
+  return same_bits(a.vs.x, b.vs.x) && same_bits(a.vs.y, b.vs.y) && same_bits(a.vs.z, b.vs.z) &&
+         same_bits(a.tsdf, b.tsdf) && a.state == b.state && max(a.recheck, 0) == max(b.recheck, 0);
+}
+
+// The march loop: kMarchMiss, kMarchZero (the sample is 0 at m.vs) or
+// kMarchBehind (the sample is behind the surface).  left: the steps left
+// before the iteration cap (those of free-space runs included).
+//
+// A fine-search ray whose signed steps return it to where it was repeats
+// itself until the iteration cap ends it without a hit: some 2700 turns in a
+// 384^3 volume, a millisecond that the whole launch waits for, on one ray in
+// ten million.  A ray still marching after kLongTurns turns (the usual one
+// takes 8, the longest regular ones about 60) goes on in the LONG form, which
+// keeps an earlier state (the one at the last power of two of its turns, R.
+// Brent, BIT 20, 1980) and ends the ray when it comes back to it.  An
+// integration and ray-cast of a 512x424 view into 384^3 that had such rays in
+// some frames took 290 to 680 us on average, and 160 us now as without them.
+//
+// Bound by instruction issue: about 65 instructions a turn and 160 a
+// free-space run, which six of eight turns compute.  The two boxes of a run
+// unrolled, the sample's nearest voxel shared with the run, reciprocal
+// approximations and the view's constants per tile took the ray-cast stage of
+// the 64-session step from 2.06 to 1.88 ms (of sixteen sessions 0.522 to
+// 0.475).  (Additions that round instead of conversions between float and
+// integer were slower, 2.21 ms: a conversion is one issue slot.)
+constexpr int kLongTurns = 64;
+template <class S, bool LONG>
+__device__ __forceinline__ int march_loop(const Vol<S>& V, F3 rd, float step_scale, float total_max, March& m, int& left) {
+  March kept = m;
+  for (int turns = 0; LONG || turns < kLongTurns; turns++) {
+    if (LONG) {
+      if (turns && same_course(m, kept)) return kMarchMiss;
+      if ((turns & (turns - 1)) == 0) kept = m;
+    }
+    if (--left < 0) return kMarchMiss;
+    float step;
+    if (m.state == COARSE)
       step = step_scale;
     else
-      step = (tsdf > 0.0f) ? fmaxf(step_scale * tsdf, 1.0f) : fminf(step_scale * tsdf, -1.0f);
-    vs = add(vs, scale(step, rd));
-    total += step;
-    if (total > total_max) break;
-    V.gtvu(vs, tsdf);
-    if (tsdf > -1.0f && tsdf < 1.0f) {
-      V.gtvi(vs, tsdf);
-      if (tsdf < 0.0f) {
-        if (state == COARSE) break;
-        state = BEHIND;
-      } else if (tsdf == 0.0f) {
-        p3d = pos_in_world(vs, s);
-        return true;
-      } else if (state == COARSE) {
-        state = FINE;
-      }
+      step = (m.tsdf > 0.0f) ? fmaxf(step_scale * m.tsdf, 1.0f) : fminf(step_scale * m.tsdf, -1.0f);
+    m.vs = add(m.vs, scale(step, rd));
+    m.total += step;
+    if (m.total > total_max) return kMarchMiss;
+    const typename Vol<S>::Near near = V.nearest(m.vs);
+    V.gtvu(near, m.tsdf);
+    if (m.tsdf > -1.0f && m.tsdf < 1.0f) {
+      V.gtvi(m.vs, m.tsdf);
+      if (m.tsdf < 0.0f) return m.state == COARSE ? kMarchMiss : kMarchBehind;
+      if (m.tsdf == 0.0f) return kMarchZero;
+      if (m.state == COARSE) m.state = FINE;
     }
-    if (tsdf == 1.0f && state != BEHIND && --recheck < 0) {
+    if (m.tsdf == 1.0f && --m.recheck < 0) {
       // While samples read TSDF 1 (no value, or a voxel whose value is 1) the
       // state and the step stay as they are, so the `run` steps of a
       // free-space run are taken at once: p + run * inc and total + run * sn.
@@ -340,32 +377,73 @@ __device__ bool cast_ray(const Vol<S>& V, const SessionDev& s, const float* K, f
       // (under 1e-2 voxel for runs of a few hundred steps and coordinates
       // below 1024), which moves the later samples and the surface point by
       // far less than the 1 mm ray-cast tolerance.
-      const float sn = (state == COARSE) ? step_scale : fmaxf(step_scale * tsdf, 1.0f);
+      const float sn = (m.state == COARSE) ? step_scale : fmaxf(step_scale * m.tsdf, 1.0f);
       const F3 inc = scale(sn, rd);
-      int m = V.free_run(vs, inc);
-      if (m < 0) {
-        recheck = -m;
-        m = 0;
+      int k = V.free_run(m.vs, inc, near);
+      if (k < 0) {
+        m.recheck = -k;
+        k = 0;
       }
-      // the loop above would stop at iteration cap + 1: run at most cap - it
+      // the loop above would stop one step past the cap: run at most `left`
       // steps here, then stop as it would.  total only grows (sn > 0), so it
       // passed total_max inside the run iff it is past it at the end, and the
       // ray then ends without a hit whichever step it was.
-      const bool capped = m > cap - it;
-      const int run = capped ? cap - it : m;
+      const bool capped = k > left;
+      const int run = capped ? left : k;
       if (run > 0) {
         const float fr = (float)run;
-        vs = add(vs, scale(fr, inc));
-        total += fr * sn;
+        m.vs = add(m.vs, scale(fr, inc));
+        m.total += fr * sn;
       }
-      if (total > total_max) return false;
-      it += run;
-      if (capped) return false;
+      if (m.total > total_max) return kMarchMiss;
+      if (capped) return kMarchMiss;
+      left -= run;
     }
   }
-  if (state == BEHIND) {
-    step = step_scale * tsdf;
-    vs = add(vs, scale(step, rd));
+  return kMarchLong;
+}
+
+// out of line: its registers are not the usual ray's
+template <class S>
+__device__ __noinline__ int march_long(const Vol<S>& V, F3 rd, float step_scale, float total_max, March& m, int left) {
+  return march_loop<S, true>(V, rd, step_scale, total_max, m, left);
+}
+
+template <class S, bool SCENE>
+__device__ bool cast_ray(const Vol<S>& V, const SessionDev& s, const TileCam& c, float px, float py, F3& p3d) {
+  const F3 pe = transform(back_project(px, py, c.K, c.dmax), c.Tcg);
+  const F3 rd = normalised(sub(pe, c.cam));
+  if (!SCENE) {
+    const float theta = acosf(dot(rd, c.ncc));
+    if (theta > c.theta_max) return false;
+  }
+  const F3 ps = add(c.cam, scale(c.dmin, rd));
+  const float step_scale = c.step_scale, total_max = c.total_max;
+  March m;
+  m.total = 0.0f;
+  m.recheck = 0;
+  pos_in_voxel(ps, s, m.vs);
+  if (!V.gtvu(V.nearest(m.vs), m.tsdf))
+    m.state = COARSE;
+  else if (m.tsdf >= 0.0f)
+    m.state = FINE;
+  else
+    return false;
+  int left = 4 * (int)total_max + 64;
+  int end = march_loop<S, false>(V, rd, step_scale, total_max, m, left);
+  if (end == kMarchLong) {
+    March far = m;
+    end = march_long<S>(V, rd, step_scale, total_max, far, left);
+    m.vs = far.vs, m.tsdf = far.tsdf;
+  }
+  if (end == kMarchZero) {
+    p3d = pos_in_world(m.vs, s);
+    return true;
+  }
+  if (end == kMarchBehind) {
+    float step = step_scale * m.tsdf;
+    F3 vs = add(m.vs, scale(step, rd));
+    float tsdf;
     V.gtvi(vs, tsdf);
     step = step_scale * tsdf;
     vs = add(vs, scale(step, rd));
@@ -375,20 +453,56 @@ __device__ bool cast_ray(const Vol<S>& V, const SessionDev& s, const float* K, f
   return false;
 }
 
-__device__ inline int ray_tiles(const SessionDev& s, int l, int rx, int ry) {
-  return ((s.lv[l].W + rx - 1) / rx) * ((s.lv[l].H + ry - 1) / ry);
+// tiles of (1 << lx) x (32 >> lx) rays of level l
+__device__ inline int ray_tiles(const SessionDev& s, int l, int lx) {
+  return ((s.lv[l].W + (1 << lx) - 1) >> lx) * ((s.lv[l].H + (32 >> lx) - 1) >> (5 - lx));
+}
+
+template <bool SCENE>
+__device__ inline void load_tile_cam(const RayArgs& a, const SessionDev& s, int l, TileCam& c) {
+  const int lane = threadIdx.x & 31;
+  const bool ext = a.level >= 0;
+  const float* Tcg = ext ? a.Tcg : s.pose->Tcg;
+  const float* Tgc = ext ? a.Tgc : s.pose->Tgc;
+  const float* cen = ext ? a.center : s.pose->center;
+  const F3 cam = f3(cen[0], cen[1], cen[2]);
+  // host-side set-up of rmi_Render_Maps_for_ICP (:1667-1675)
+  const F3 cc = f3(s.cube_center[0], s.cube_center[1], s.cube_center[2]);
+  const F3 vcc = sub(cc, cam);
+  const F3 ncc = normalised(vcc);
+  const float dist_cc = length(vcc);
+  const float theta_max = asinf(s.r_cube / dist_cc);
+  __syncwarp();  // the previous tile's rays have read theirs
+  if (lane < 12) c.Tcg[lane] = Tcg[lane], c.Tgc[lane] = Tgc[lane];
+  if (lane < 4) c.K[lane] = s.lv[l].K[lane];
+  if (lane == 0) {
+    c.cam = cam;
+    c.theta_max = theta_max;
+    c.ncc = ncc;
+    // object mode (d_crtc_NEW, :466-635): the segment of the ray through the
+    // cube's bounding sphere inside its view cone; scene mode (d_crtcs,
+    // :908-1066): from the camera centre to 2 r_cube, no cone
+    c.dmin = SCENE ? 0.0f : dist_cc - s.r_cube;
+    c.dmax = SCENE ? 2.0f * s.r_cube : dist_cc + s.r_cube;
+    c.step_scale = 0.9f * s.mu * s.vox_inv;
+    c.total_max = 2.0f * s.r_cube * s.vox_inv;
+  }
+  __syncwarp();
 }
 
 // Hands the calling warp ray tiles until none are left and calls
-// f(session, level, x, y) for each lane's pixel inside its level.  The last
-// warp to finish clears the counters for the next launch.
-template <class F>
+// f(session, level, x, y, camera) for each lane's pixel inside its level.  The
+// last warp to finish clears the counters for the next launch.
+template <bool SCENE, class F>
 __device__ inline void for_each_ray_tile(const RayArgs& a, F&& f) {
+  __shared__ TileCam cams[kRayThreads / 32];
+  TileCam& cam = cams[threadIdx.x >> 5];
   const BatchTable* __restrict__ bt = a.bt;
   const int lane = threadIdx.x & 31;
   const int n = bt->n;
-  const int lx = bt->ray_lx, rx = 1 << lx, ry = 32 >> lx;
-  const int total = (a.level >= 0) ? ray_tiles(*bt->s[0], a.level, rx, ry) : bt->ray[n];
+  const int lx = bt->ray_lx, rx = 1 << lx;
+  const int total = (a.level >= 0) ? ray_tiles(*bt->s[0], a.level, lx) : bt->ray[n];
+  int loaded = -1;  // slot and level of cam
   for (;;) {
     int item = 0;
     if (lane == 0) item = (int)atomicAdd(a.work, 1u);
@@ -404,16 +518,20 @@ __device__ inline void for_each_ray_tile(const RayArgs& a, F&& f) {
       const SessionDev& s = *bt->s[slot];
       l = 0;
       for (; l < s.levels - 1; l++) {
-        const int nt = ray_tiles(s, l, rx, ry);
+        const int nt = ray_tiles(s, l, lx);
         if (t < nt) break;
         t -= nt;
       }
     }
     const SessionDev& s = *bt->s[slot];
     if (a.gate && s.pose->failed) continue;
-    const int tw = (s.lv[l].W + rx - 1) / rx;
-    const int x = (t % tw) * rx + (lane & (rx - 1)), y = (t / tw) * ry + (lane >> lx);
-    if (x < s.lv[l].W && y < s.lv[l].H) f(s, l, x, y);
+    if (loaded != slot * kMaxLevels + l) {
+      loaded = slot * kMaxLevels + l;
+      load_tile_cam<SCENE>(a, s, l, cam);
+    }
+    const int tw = (s.lv[l].W + rx - 1) >> lx, ty = t / tw;
+    const int x = ((t - ty * tw) << lx) + (lane & (rx - 1)), y = (ty << (5 - lx)) + (lane >> lx);
+    if (x < s.lv[l].W && y < s.lv[l].H) f(s, l, x, y, cam);
   }
   if (lane == 0) {
     __threadfence();
@@ -438,7 +556,7 @@ __device__ inline Vol<S> volume_of(const SessionDev& s) {
   Vol<S> V;
   V.v = reinterpret_cast<const typename S::word*>(s.vol);
   V.bdist = s.bdist;
-  for (int k = 0; k < 3; k++) V.dim[k] = s.dim[k];
+  for (int k = 0; k < 3; k++) V.dim[k] = (float)s.dim[k];
   V.nbx = (uint32_t)s.nb[0];
   V.nbxy = (uint32_t)s.nb[0] * (uint32_t)s.nb[1];
   V.sy = (uint32_t)s.nb[0] << 9;
@@ -532,40 +650,13 @@ __global__ void __launch_bounds__(kBandThreads) k_band_z(const BatchTable* __res
 #define VS_SHADE_MIN_BLOCKS 8
 #endif
 
-// the ray of pixel (x, y) of level l to its surface point pg (global
-// coordinates); false: no hit
-template <class S, bool SCENE>
-__device__ inline bool march_ray(const RayArgs& a, const Vol<S>& V, const SessionDev& s, int l, int x, int y, F3& pg) {
-  const bool ext = a.level >= 0;
-  const float* Tcg_in = ext ? a.Tcg : s.pose->Tcg;
-  const float* cen = ext ? a.center : s.pose->center;
-  float Tcg[12], K[4];
-#pragma unroll
-  for (int k = 0; k < 12; k++) Tcg[k] = Tcg_in[k];
-#pragma unroll
-  for (int k = 0; k < 4; k++) K[k] = s.lv[l].K[k];
-  const F3 cam = f3(cen[0], cen[1], cen[2]);
-  // host-side set-up of rmi_Render_Maps_for_ICP (:1667-1675)
-  const F3 cc = f3(s.cube_center[0], s.cube_center[1], s.cube_center[2]);
-  const F3 vcc = sub(cc, cam);
-  const F3 ncc = normalised(vcc);
-  const float dist_cc = length(vcc);
-  const float theta_max = asinf(s.r_cube / dist_cc);
-  // object mode (d_crtc_NEW, :466-635): the segment of the ray through the
-  // cube's bounding sphere inside its view cone; scene mode (d_crtcs,
-  // :908-1066): from the camera centre to 2 r_cube, no cone
-  const float dmin = SCENE ? 0.0f : dist_cc - s.r_cube;
-  const float dmax = SCENE ? 2.0f * s.r_cube : dist_cc + s.r_cube;
-  return cast_ray(V, s, K, (float)x, (float)y, Tcg, cam, dmin, dmax, !SCENE, ncc, theta_max, pg);
-}
-
 // phase 1: march every ray to its surface point (global coordinates; w = 1
 // hit, 0 none) in the session's hit buffer
 template <class S, bool SCENE>
 __global__ void __launch_bounds__(kRayThreads, VS_RAY_MIN_BLOCKS) k_ray_march(RayArgs a) {
-  for_each_ray_tile(a, [&](const SessionDev& s, int l, int x, int y) {
+  for_each_ray_tile<SCENE>(a, [&](const SessionDev& s, int l, int x, int y, const TileCam& c) {
     F3 pg;
-    const bool hit = march_ray<S, SCENE>(a, volume_of<S>(s), s, l, x, y, pg);
+    const bool hit = cast_ray<S, SCENE>(volume_of<S>(s), s, c, (float)x, (float)y, pg);
     s.ray_hit[hit_offset(s, l) + (size_t)y * s.lv[l].W + x] =
         hit ? make_float4(pg.x, pg.y, pg.z, 1.0f) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   });
@@ -585,8 +676,8 @@ __device__ uint32_t trilinear_color(const Vol<S>& V, const SessionDev& s, F3 pg)
   const int ox = (int)fx, oy = (int)fy, oz = (int)fz;
   const float rx = v.x - fx, ry = v.y - fy, rz = v.z - fz;
   float tdummy;
-  bool ok = ox >= 0 && ox + 1 < V.dim[0] && oy >= 0 && oy + 1 < V.dim[1] && oz >= 0 && oz + 1 < V.dim[2];
-  const int cx = min(max(ox, 0), V.dim[0] - 2), cy = min(max(oy, 0), V.dim[1] - 2), cz = min(max(oz, 0), V.dim[2] - 2);
+  bool ok = ox >= 0 && ox + 1 < s.dim[0] && oy >= 0 && oy + 1 < s.dim[1] && oz >= 0 && oz + 1 < s.dim[2];
+  const int cx = min(max(ox, 0), s.dim[0] - 2), cy = min(max(oy, 0), s.dim[1] - 2), cz = min(max(oz, 0), s.dim[2] - 2);
   const uint32_t X[2] = {V.wx(cx), V.wx(cx + 1)}, Y[2] = {V.wy(cy), V.wy(cy + 1)}, Z[2] = {V.wz(cz), V.wz(cz + 1)};
   uint32_t c[8];
 #pragma unroll
@@ -625,7 +716,7 @@ __device__ uint32_t nearest_color(const Vol<S>& V, const SessionDev& s, F3 pg) {
   pos_in_voxel(pg, s, v);
   if (isnan(v.x) || isnan(v.y) || isnan(v.z)) return 0u;
   const int x = roundf_ref(v.x), y = roundf_ref(v.y), z = roundf_ref(v.z);
-  if (x < 0 || x >= V.dim[0] || y < 0 || y >= V.dim[1] || z < 0 || z >= V.dim[2]) return 0u;
+  if (x < 0 || x >= s.dim[0] || y < 0 || y >= s.dim[1] || z < 0 || z >= s.dim[2]) return 0u;
   const uint32_t w = V.wx(x) + V.wy(y) + V.wz(z);
   float t;
   if (!V.word_ok(w, t)) return 0u;
@@ -635,8 +726,8 @@ __device__ uint32_t nearest_color(const Vol<S>& V, const SessionDev& s, F3 pg) {
 // surface normal of a hit (d_csnt), camera-frame vertex and normal, shading,
 // colour, into the model maps or the external outputs
 template <class S, bool COLOR>
-__device__ inline void shade_ray(const RayArgs& a, const Vol<S>& V, const SessionDev& s, int l, int x, int y,
-                                 bool hit, F3 pg) {
+__device__ inline void shade_ray(const RayArgs& a, const Vol<S>& V, const SessionDev& s, const TileCam& c, int l,
+                                 int x, int y, bool hit, F3 pg) {
   const bool ext = a.level >= 0;
   const size_t idx = (size_t)y * s.lv[l].W + x;
   F3 sn;
@@ -647,13 +738,9 @@ __device__ inline void shade_ray(const RayArgs& a, const Vol<S>& V, const Sessio
   F3 pc = f3(-100.0f, -100.0f, -100.0f), sc = f3(-100.0f, -100.0f, -100.0f);
   if (valid) {
     if (COLOR && s.col) rgb = (a.mode & kRayNearestColor) ? nearest_color(V, s, pg) : trilinear_color(V, s, pg);
-    const float* Tgc_in = ext ? a.Tgc : s.pose->Tgc;
-    float Tgc[12];
-#pragma unroll
-    for (int k = 0; k < 12; k++) Tgc[k] = Tgc_in[k];
-    pc = transform(pg, Tgc);
+    pc = transform(pg, c.Tgc);
     dep = pc.z;
-    sc = (a.mode & kRayGlobalNormals) ? sn : rotate(sn, Tgc);
+    sc = (a.mode & kRayGlobalNormals) ? sn : rotate(sn, c.Tgc);
     float ang = sc.x * a.light[0] + sc.y * a.light[1] + sc.z * a.light[2];
     img = fmaxf(0.0f, fminf(255.0f, (0.8f * ang + 0.2f) * 255.0f));
   }
@@ -688,9 +775,9 @@ __device__ inline void shade_ray(const RayArgs& a, const Vol<S>& V, const Sessio
 // phase 2: the maps of every ray from its surface point in the hit buffer
 template <class S, bool COLOR>
 __global__ void __launch_bounds__(kRayThreads, VS_SHADE_MIN_BLOCKS) k_ray_shade(RayArgs a) {
-  for_each_ray_tile(a, [&](const SessionDev& s, int l, int x, int y) {
+  for_each_ray_tile<false>(a, [&](const SessionDev& s, int l, int x, int y, const TileCam& c) {
     const float4 h = s.ray_hit[hit_offset(s, l) + (size_t)y * s.lv[l].W + x];
-    shade_ray<S, COLOR>(a, volume_of<S>(s), s, l, x, y, h.w != 0.0f, f3(h.x, h.y, h.z));
+    shade_ray<S, COLOR>(a, volume_of<S>(s), s, c, l, x, y, h.w != 0.0f, f3(h.x, h.y, h.z));
   });
 }
 
@@ -702,11 +789,11 @@ __global__ void __launch_bounds__(kRayThreads, VS_SHADE_MIN_BLOCKS) k_ray_shade(
 // colour)
 template <class S, bool SCENE>
 __global__ void __launch_bounds__(kRayThreads, VS_FUSED_MIN_BLOCKS) k_ray_fused(RayArgs a) {
-  for_each_ray_tile(a, [&](const SessionDev& s, int l, int x, int y) {
+  for_each_ray_tile<SCENE>(a, [&](const SessionDev& s, int l, int x, int y, const TileCam& c) {
     const Vol<S> V = volume_of<S>(s);
     F3 pg;
-    const bool hit = march_ray<S, SCENE>(a, V, s, l, x, y, pg);
-    shade_ray<S, false>(a, V, s, l, x, y, hit, pg);
+    const bool hit = cast_ray<S, SCENE>(V, s, c, (float)x, (float)y, pg);
+    shade_ray<S, false>(a, V, s, c, l, x, y, hit, pg);
   });
 }
 

@@ -167,6 +167,14 @@ __host__ __device__ inline F3 normalised(F3 a) {
   float inv = 1.0f / sqrtf(a.x * a.x + a.y * a.y + a.z * a.z);
   return f3(a.x * inv, a.y * inv, a.z * inv);
 }
+// rcp.approx.ftz.f32: the reciprocal with at most 1 ulp of error (PTX ISA,
+// "rcp.approx"), one special-function instruction
+__device__ __forceinline__ float rcp_approx(float z) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(z));
+  return r;
+}
+
 // d_p_Project (_yooji_cuda_math.h:205-210)
 __host__ __device__ inline void project(F3 p, const float* K, float& u, float& v) {
   u = K[0] * p.x / p.z + K[2];
@@ -247,8 +255,10 @@ __device__ inline int tsdf_to_q(float t) {
 
 struct StoreI16 {
   typedef uint32_t word;
+  __device__ static inline float value(word v) { return q_to_tsdf((int)(int16_t)(v & 0xffffu)); }
+  __device__ static inline bool weighted(word v) { return v >= 0x10000u; }
   __device__ static inline void decode(word v, float& t, uint32_t& w) {
-    t = q_to_tsdf((int)(int16_t)(v & 0xffffu));
+    t = value(v);
     w = v >> 16;
   }
   __device__ static inline word encode(float t, uint32_t w) {
@@ -260,8 +270,12 @@ struct StoreI16 {
 };
 struct StoreF16 {
   typedef uint32_t word;
+  __device__ static inline float value(word v) {
+    return __half2float(__ushort_as_half((unsigned short)(v & 0xffffu)));
+  }
+  __device__ static inline bool weighted(word v) { return v >= 0x10000u; }
   __device__ static inline void decode(word v, float& t, uint32_t& w) {
-    t = __half2float(__ushort_as_half((unsigned short)(v & 0xffffu)));
+    t = value(v);
     w = v >> 16;
   }
   __device__ static inline word encode(float t, uint32_t w) {
@@ -272,6 +286,8 @@ struct StoreF16 {
 };
 struct StoreF32 {
   typedef uint2 word;
+  __device__ static inline float value(word v) { return __uint_as_float(v.x); }
+  __device__ static inline bool weighted(word v) { return v.y != 0u; }
   __device__ static inline void decode(word v, float& t, uint32_t& w) {
     t = __uint_as_float(v.x);
     w = v.y;
