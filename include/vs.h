@@ -415,8 +415,9 @@ int vs_batch_kernels_per_step(vs_batch* b);
  * grid (march and shading in one launch; colour sessions: the march grid,
  * then the shading grid) holds that many 128-thread blocks per SM (0: as
  * many as fit);
- * the bilateral filter and the sub-cube activation work on 32 x
- * bilateral_rows pixel tiles (4, 8 or 16; 0: 8); the integration's update
+ * the bilateral filter works on tiles of 32 x twice bilateral_rows pixels and
+ * the sub-cube activation on 32 x bilateral_rows (4, 8 or 16; 0: 8); the
+ * integration's update
  * grid holds integrate_blocks_per_sm 256-thread blocks per SM (0: as many as
  * fit).  The shape changes no result, only time. */
 typedef struct {

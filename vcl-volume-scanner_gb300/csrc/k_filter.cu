@@ -18,78 +18,178 @@
 namespace vs {
 namespace {
 
-constexpr int BX = 32, BY = 8;  // output tile of the bilateral filter (BY: default rows; 4 and 16 also built)
+constexpr int BX = 32, BY = 8;  // threads of a filter block (BY: default rows; 4 and 16 also built)
+constexpr int kPerThread = 2;   // outputs per thread, consecutive rows
 constexpr int kScanSmem = 64 * 1024;  // staged normal-rejection bitmasks of one level
 
 // The reference reads a linear-filtered texture at integer coordinates, so
 // every tap is the mean of the 2x2 texels (X-1..X, Y-1..Y); out-of-range texel
-// coordinates clamp to the edge.  A tile of BX x BY outputs needs taps
+// coordinates clamp to the edge.  A tile of BX x 2R outputs needs taps
 // X in [x0-2, x0+BX+1] and texels in [x0-3, x0+BX+1].
+//
+// Bound by the 24 exponentials of a pixel on the special-function unit (an
+// eighth of a warp per cycle and scheduler: 192 cycles per warp and row) and
+// as much by its other instructions (eight per tap).  A thread filters
+// consecutive rows of a column, so taps are read from shared memory 15 times
+// per pixel instead of 25 and the tile's borders shrink, and holes need no
+// test per tap.  With one output per thread in 32 x 8 tiles 1920x1080 took
+// 33.5 us, and takes 25.2; four rows per thread 26 us, and 2 us more for one
+// 640x480 frame, whose tiles are few.
 template <int R>
 struct BilateralSmem {
-  float tex[R + 5][BX + 6];
-  float tap[R + 4][BX + 5];
+  float tex[kPerThread * R + 5][BX + 6];
+  float tap[kPerThread * R + 4][BX + 5];
 };
 
-template <int R>
-__device__ inline float bilateral_px(const BilateralSmem<R>& m, int tx, int ty, const float g[5]) {
-  // The reference's exponent is -mod / (2 sigma_r^2), 2 sigma_r^2 = 2.0f *
-  // 0.1f * 0.1f with sigma_r = 0.1 m (z_yooji_cuda_img_proc.cu:44,91).  Here
-  // it is the product with the folded constant -1 / (2 sigma_r^2): one
-  // rounding more than the quotient (a relative 1.2e-7 of an exponent that
-  // matters only below ~20), far inside the 1e-5 m tolerance of the filtered
-  // depth, and no division per tap.
-  constexpr float kNegInvDenom = -1.0f / (2.0f * 0.1f * 0.1f);
-  const float center = m.tap[ty + 2][tx + 2];
-  float t = 0.0f, sum = 0.0f;
-#pragma unroll
-  for (int i = -2; i <= 2; i++) {
-#pragma unroll
-    for (int j = -2; j <= 2; j++) {
-      float cur = m.tap[ty + 2 + i][tx + 2 + j];
-      if (cur <= 0.0f) return 0.0f;
-      float mod = (center - cur) * (center - cur);
-      float factor = g[i + 2] * g[j + 2] * __expf(mod * kNegInvDenom);
-      t += factor * cur;
-      sum += factor;
-    }
-  }
-  return t / sum;
+// exp2 by the special-function unit (ex2.approx.ftz.f32)
+__device__ __forceinline__ float exp2_approx(float x) {
+  float r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
 }
 
-// one BX x R output tile; the block's BX x R threads all take part (two barriers)
+// The filter of kPerThread pixels, rows ty0 .. of column tx.  Every sum runs in
+// the reference's order with its roundings.  A tap that is not above 0 is stored as
+// -infinity: as the centre it makes the sum infinite, elsewhere its weight is
+// 0 and their product not a number.
+template <int R>
+__device__ inline void bilateral_px(const BilateralSmem<R>& m, int tx, int ty0, bool finite, float out[kPerThread]) {
+  // The Gaussian of delta 4 (:275-286), exp(-x^2 / (2 * 4^2)).  The range
+  // weight's exponent is -mod / (2 sigma_r^2), 2 sigma_r^2 = 2.0f * 0.1f *
+  // 0.1f with sigma_r = 0.1 m (z_yooji_cuda_img_proc.cu:44,91), here the
+  // product with the folded constant -1 / (2 sigma_r^2): one rounding more
+  // than the quotient (a relative 1.2e-7 of an exponent that matters only
+  // below ~20), far inside the 1e-5 m tolerance of the filtered depth, and no
+  // division per tap.  Its exponential is that of the product with log2(e) to
+  // the base 2; below 2^-126 it gives 0, which no sum of weights that holds
+  // the centre's 1 tells from the subnormal.
+  constexpr float g1 = 0.96923321f, g2 = 0.88249689f;  // exp(-1 / 32), exp(-4 / 32) rounded to float
+  constexpr float g[5] = {g2, g1, 1.0f, g1, g2};
+  constexpr float kNegInvDenom = -1.0f / (2.0f * 0.1f * 0.1f), kLog2e = 1.44269504f;
+  float c[kPerThread], t[kPerThread], sum[kPerThread];
+#pragma unroll
+  for (int r = 0; r < kPerThread; r++) {
+    c[r] = m.tap[ty0 + r + 2][tx + 2];
+    t[r] = sum[r] = 0.0f;
+  }
+#pragma unroll
+  for (int k = 0; k < kPerThread + 4; k++) {
+    float a[5];
+#pragma unroll
+    for (int j = 0; j < 5; j++) a[j] = m.tap[ty0 + k][tx + j];
+#pragma unroll
+    for (int r = 0; r < kPerThread; r++) {
+      const int i = k - r;
+      if (i < 0 || i > 4) continue;
+#pragma unroll
+      for (int j = 0; j < 5; j++) {
+        if (i == 2 && j == 2) {  // the centre: weight 1
+          t[r] += c[r];
+          sum[r] += 1.0f;
+          continue;
+        }
+        const float d = c[r] - a[j];
+        const float w = (g[i] * g[j]) * exp2_approx(d * d * kNegInvDenom * kLog2e);
+        t[r] += w * a[j];
+        sum[r] += w;
+      }
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < kPerThread; r++) {
+    out[r] = t[r] / sum[r];
+    if (!(t[r] >= 0.0f)) {
+      bool hole = finite;  // finite inputs: only a hole gives this
+      if (!finite)
+        for (int i = 0; i < 25; i++) hole |= m.tap[ty0 + r + i / 5][tx + i % 5] == __int_as_float(0xff800000);
+      if (hole) out[r] = 0.0f;
+    }
+  }
+}
+
+// one BX x 2R output tile; the block's BX x R threads all take part (two barriers)
 template <bool FROM_MM, int R>
 __device__ inline void bilateral_tile(BilateralSmem<R>& m, const uint16_t* __restrict__ mm,
                                       const float* __restrict__ fin, float scale, float* __restrict__ raw_out,
-                                      float* __restrict__ out, int W, int H, int x0, int y0, const float g[5],
+                                      float* __restrict__ out, int W, int H, int x0, int y0,
                                       float2* __restrict__ dl_out = nullptr, const float* __restrict__ lam = nullptr) {
-  const int tid = threadIdx.y * BX + threadIdx.x;
-  for (int i = tid; i < (R + 5) * (BX + 5); i += BX * R) {
-    int ty = i / (BX + 5), tx = i - ty * (BX + 5);
-    int gx = min(max(x0 - 3 + tx, 0), W - 1);
-    int gy = min(max(y0 - 3 + ty, 0), H - 1);
-    float v;
-    if (FROM_MM)
-      v = (float)mm[(size_t)gy * W + gx] * scale;
-    else
-      v = fin[(size_t)gy * W + gx];
-    m.tex[ty][tx] = v;
-  }
-  __syncthreads();
-  for (int i = tid; i < (R + 4) * (BX + 4); i += BX * R) {
-    int ty = i / (BX + 4), tx = i - ty * (BX + 4);
-    m.tap[ty][tx] = 0.25f * ((m.tex[ty][tx] + m.tex[ty][tx + 1]) + (m.tex[ty + 1][tx] + m.tex[ty + 1][tx + 1]));
-  }
-  __syncthreads();
+  constexpr int TR = kPerThread * R;
   const int tx = threadIdx.x, ty = threadIdx.y;
-  const int x = x0 + tx, y = y0 + ty;
-  if (x < W && y < H) {
-    if (FROM_MM) {
-      const float raw = m.tex[ty + 3][tx + 3];
-      raw_out[(size_t)y * W + x] = raw;
-      if (dl_out) dl_out[(size_t)y * W + x] = make_float2(raw, __ldg(lam + (size_t)y * W + x));
+  // a warp per texel row: BX columns, then the five beyond
+#pragma unroll
+  for (int q = 0; q < (TR + 5 + R - 1) / R; q++) {
+    const int r = ty + q * R;
+    if (r < TR + 5) {
+      const int gy = min(max(y0 - 3 + r, 0), H - 1);
+      const int gx = min(max(x0 - 3 + tx, 0), W - 1), gx2 = min(max(x0 - 3 + BX + tx, 0), W - 1);
+      if (FROM_MM) {
+        m.tex[r][tx] = (float)mm[(size_t)gy * W + gx] * scale;
+        if (tx < 5) m.tex[r][BX + tx] = (float)mm[(size_t)gy * W + gx2] * scale;
+      } else {
+        m.tex[r][tx] = fin[(size_t)gy * W + gx];
+        if (tx < 5) m.tex[r][BX + tx] = fin[(size_t)gy * W + gx2];
+      }
     }
-    out[(size_t)y * W + x] = bilateral_px(m, tx, ty, g);
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < (TR + 4 + R - 1) / R; q++) {
+    const int r = ty + q * R;
+    if (r < TR + 4) {
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        const int x = tx + e * BX;
+        if (e == 0 || tx < 4) {
+          const float v = 0.25f * ((m.tex[r][x] + m.tex[r][x + 1]) + (m.tex[r + 1][x] + m.tex[r + 1][x + 1]));
+          m.tap[r][x] = v <= 0.0f ? __int_as_float(0xff800000) : v;
+        }
+      }
+    }
+  }
+  __syncthreads();
+  const int x = x0 + tx, yb = y0 + ty * kPerThread;
+  if (x < W && yb < H) {
+    float f[kPerThread];
+    bilateral_px(m, tx, ty * kPerThread, FROM_MM, f);
+#pragma unroll
+    for (int r = 0; r < kPerThread; r++) {
+      if (yb + r >= H) break;
+      const size_t i = (size_t)(yb + r) * W + x;
+      if (FROM_MM) {
+        const float raw = m.tex[ty * kPerThread + r + 3][tx + 3];
+        raw_out[i] = raw;
+        if (dl_out) dl_out[i] = make_float2(raw, __ldg(lam + i));
+      }
+      out[i] = f[r];
+    }
+  }
+}
+
+// Frames read in place (device memory, or pinned host memory over the host
+// link) into the sessions' frame buffers: each pixel crosses the link once, in
+// 8-byte reads.  (The filter reading such a frame itself read every pixel 2.9
+// times with its tiles' borders: the filter stage of the 64-session step from
+// pinned frames took 0.98 ms, and takes 0.70.)  A slot's filter tiles count its
+// chunks of 2 BX BY pixels: they cover the image, so the chunks do.
+__global__ void __launch_bounds__(BX* BY) k_ingest(const BatchTable* __restrict__ bt) {
+  const int n = bt->n;
+  const int total = bt->fil[n];
+  for (int item = blockIdx.x; item < total; item += gridDim.x) {
+    int t;
+    const int slot = find_slot(bt->fil, n, item, t);
+    const SessionDev* __restrict__ s = bt->s[slot];
+    const uint16_t* __restrict__ src = bt->frame[slot];
+    if (!src || src == s->depth_mm) continue;
+    uint16_t* __restrict__ dst = s->depth_mm;
+    const int px = s->lv[0].W * s->lv[0].H, chunk = kPerThread * BX * bt->bil_rows;
+    const bool wide = (reinterpret_cast<uintptr_t>(src) & 7) == 0;
+    for (int i = t * chunk + threadIdx.x * 4; i < min(px, (t + 1) * chunk); i += BX * BY * 4) {
+      if (wide && i + 4 <= px) {
+        *reinterpret_cast<uint2*>(dst + i) = *reinterpret_cast<const uint2*>(src + i);
+      } else {
+        for (int k = i; k < min(px, i + 4); k++) dst[k] = src[k];
+      }
+    }
   }
 }
 
@@ -97,26 +197,20 @@ template <int R>
 __global__ void __launch_bounds__(BX* R) k_bilateral_batch(const BatchTable* __restrict__ bt) {
   __shared__ BilateralSmem<R> m;
   const int n = bt->n;
-  const int total = bt->bil[n];
+  const int total = bt->fil[n];
   for (int item = blockIdx.x; item < total; item += gridDim.x) {
     int t;
-    const int slot = find_slot(bt->bil, n, item, t);
+    const int slot = find_slot(bt->fil, n, item, t);
     const SessionDev* __restrict__ s = bt->s[slot];
     const int W = s->lv[0].W, H = s->lv[0].H;
-    const int tw = (W + BX - 1) / BX;
-    const float g[5] = {s->gauss[0], s->gauss[1], s->gauss[2], s->gauss[1], s->gauss[0]};
-    const uint16_t* __restrict__ mm = bt->frame[slot] ? bt->frame[slot] : s->depth_mm;
-    bilateral_tile<true, R>(m, mm, nullptr, s->depth_scale, s->depth_raw, s->depth[0], W, H, (t % tw) * BX,
-                            (t / tw) * R, g, s->lam_map ? s->dl_map : nullptr, s->lam_map);
-    if (mm != s->depth_mm) {
-      // a frame read in place: the session's own frame buffer is kept current
-      const int x = (t % tw) * BX + threadIdx.x, y = (t / tw) * R + threadIdx.y;
-      if (x < W && y < H) s->depth_mm[(size_t)y * W + x] = mm[(size_t)y * W + x];
-    }
+    const int tw = (W + BX - 1) / BX, tyy = t / tw;
+    const int x0 = (t - tyy * tw) * BX, y0 = tyy * R * kPerThread;
+    bilateral_tile<true, R>(m, s->depth_mm, nullptr, s->depth_scale, s->depth_raw, s->depth[0], W, H, x0, y0,
+                            s->lam_map ? s->dl_map : nullptr, s->lam_map);
     if (s->rgb_packed) {
       // the colour frame as one word per pixel, for the integration's gathers
-      const int x = (t % tw) * BX + threadIdx.x, y = (t / tw) * R + threadIdx.y;
-      if (x < W && y < H) {
+      const int x = x0 + threadIdx.x;
+      for (int y = y0 + threadIdx.y; x < W && y < min(H, y0 + R * kPerThread); y += R) {
         const size_t i = (size_t)y * W + x, plane = (size_t)W * H;
         s->rgb_packed[i] = pack_rgb(s->rgb_in[i], s->rgb_in[plane + i], s->rgb_in[2 * plane + i]);
       }
@@ -125,12 +219,10 @@ __global__ void __launch_bounds__(BX* R) k_bilateral_batch(const BatchTable* __r
   }
 }
 
-__global__ void __launch_bounds__(BX* BY)
-    k_bilateral_float(const float* __restrict__ in, float* __restrict__ out, int W, int H, float g0, float g1,
-                      float g2) {
+__global__ void __launch_bounds__(BX* BY, 6)
+    k_bilateral_float(const float* __restrict__ in, float* __restrict__ out, int W, int H) {
   __shared__ BilateralSmem<BY> m;
-  const float g[5] = {g0, g1, g2, g1, g0};
-  bilateral_tile<false, BY>(m, nullptr, in, 1.0f, nullptr, out, W, H, blockIdx.x * BX, blockIdx.y * BY, g);
+  bilateral_tile<false, BY>(m, nullptr, in, 1.0f, nullptr, out, W, H, blockIdx.x * BX, blockIdx.y * BY * kPerThread);
 }
 
 // level l -> l+1: separable [1 4 6 4 1] smoothing (borders 0, no validity
@@ -494,8 +586,9 @@ __global__ void __launch_bounds__(256) k_inmap_post(const BatchTable* __restrict
 
 }  // namespace
 
-void launch_filter(const BatchTable* bt, cudaStream_t st, int rows) {
+void launch_filter(const BatchTable* bt, cudaStream_t st, int rows, bool ingest) {
   const int grid = sm_count() * 8;
+  if (ingest) k_ingest<<<grid, BX * BY, 0, st>>>(bt);
   switch (rows) {
     case 4:
       k_bilateral_batch<4><<<grid * 2, dim3(BX, 4), 0, st>>>(bt);
@@ -519,8 +612,8 @@ void launch_input_maps(const BatchTable* bt, cudaStream_t st) {
 
 void launch_bilateral_float(const SessionDev& h, const float* in, float* out, cudaStream_t st) {
   const int W = h.lv[0].W, H = h.lv[0].H;
-  dim3 blk(BX, BY), grd((W + BX - 1) / BX, (H + BY - 1) / BY);
-  k_bilateral_float<<<grd, blk, 0, st>>>(in, out, W, H, h.gauss[0], h.gauss[1], h.gauss[2]);
+  dim3 blk(BX, BY), grd((W + BX - 1) / BX, (H + BY * kPerThread - 1) / (BY * kPerThread));
+  k_bilateral_float<<<grd, blk, 0, st>>>(in, out, W, H);
 }
 
 void configure_filter_kernels() {
@@ -547,6 +640,8 @@ void fill_batch_table(BatchTable& hb, const SessionDev* const* host_recs, const 
       ray += ((w + rx - 1) / rx) * ((hh + ry - 1) / ry);
     }
     hb.bil[i + 1] = hb.bil[i] + ((h.lv[0].W + BX - 1) / BX) * ((h.lv[0].H + hb.bil_rows - 1) / hb.bil_rows);
+    const int fr = hb.bil_rows * kPerThread;
+    hb.fil[i + 1] = hb.fil[i] + ((h.lv[0].W + BX - 1) / BX) * ((h.lv[0].H + fr - 1) / fr);
     for (int l = 1; l < kMaxLevels; l++)
       hb.pyr[l - 1][i + 1] =
           hb.pyr[l - 1][i] + (l < h.levels ? ((h.lv[l].W + 31) / 32) * ((h.lv[l].H + 7) / 8) : 0);

@@ -110,12 +110,6 @@ void fill_geometry(const vs_config* c, SessionDev& h) {
   h.reduce_mode = c->reduce_mode;
   h.tsdf_type = c->tsdf_type;
   h.depth_scale = c->depth_scale;
-  // cGaussian (updateGaussian, z_yooji_cuda_img_proc.cu:275-286), delta 4, radius 2
-  const float delta = 4.0f;
-  for (int i = 0; i < 5; i++) {
-    float x = (float)(i - 2);
-    h.gauss[i] = std::exp(-(x * x) / (2 * delta * delta));
-  }
 }
 
 template <class T>

@@ -91,7 +91,7 @@ void drop_graphs(vs_batch* b) {
 // one group's per-frame chain on one stream
 void record_chain(vs_batch* b, const BatchTable* t, cudaStream_t st) {
   const Schedule& k = b->sched;
-  launch_filter(t, st, b->shape.bil_rows);
+  launch_filter(t, st, b->shape.bil_rows, true);
   if (k.inmaps) launch_input_maps(t, st);
   launch_icp(t, k.reduce_mode, st, true, nullptr);
   launch_integrate(t, k.tsdf_type, nullptr, nullptr, nullptr, true, st, k.color != 0, b->shape.integrate_blocks_per_sm);
@@ -120,7 +120,7 @@ void record_step(vs_batch* b, int r, cudaStream_t st) {
     // stage timing: the stages one after another (ICP still on branches), so
     // that each stage's time is its own
     mark(0);
-    launch_filter(b->d_tab, st, b->shape.bil_rows);
+    launch_filter(b->d_tab, st, b->shape.bil_rows, true);
     if (k.inmaps) launch_input_maps(b->d_tab, st);
     mark(1);
     cudaEventRecord(b->fork, st);

@@ -61,7 +61,6 @@ struct SessionDev {
   int iters[kMaxLevels];
   int reduce_mode, tsdf_type;
   float depth_scale;
-  float gauss[5];       // bilateral spatial weights
   // frame buffers
   uint16_t* depth_mm;            // level-0 input (uint16)
   float* depth_raw;              // level-0 metres (integration input)
@@ -120,7 +119,8 @@ struct BatchTable {
   int ray_lx;                          // ray tile of a warp: (1 << ray_lx) x (32 >> ray_lx) rays
   int bil_rows;                        // rows of a level-0 tile (bilateral, activation): 4, 8 or 16
   const SessionDev* s[kMaxSlots];
-  int bil[kMaxSlots + 1];              // level-0 32 x bil_rows tiles (bilateral, activation)
+  int bil[kMaxSlots + 1];              // level-0 32 x bil_rows tiles (activation)
+  int fil[kMaxSlots + 1];              // level-0 32 x 2 bil_rows tiles (ingest, bilateral)
   int pyr[kMaxLevels - 1][kMaxSlots + 1];  // 32x8 tiles of levels 1, 2
   int imap[kMaxSlots + 1];             // input-map 32x32 tiles, all levels
   int scan[kMaxSlots + 1];             // input-map row scans: one per level
@@ -320,7 +320,8 @@ int sm_count();
 void fill_batch_table(BatchTable& hb, const SessionDev* const* host_recs, const SessionDev* const* dev_recs, int n,
                       int ray_lx = 3, int bil_rows = 8);
 int ray_max_blocks_per_sm(int tsdf_type, bool shade);
-void launch_filter(const BatchTable* bt, cudaStream_t st, int bil_rows = 8);
+// ingest: some slot's frame may be read in place (BatchTable::frame)
+void launch_filter(const BatchTable* bt, cudaStream_t st, int bil_rows = 8, bool ingest = false);
 void launch_input_maps(const BatchTable* bt, cudaStream_t st);
 void launch_bilateral_float(const SessionDev& h, const float* in, float* out, cudaStream_t st);
 // ICP of every slot, each session through its own levels and iterations
