@@ -13,9 +13,17 @@
 // stores it), 0 where none lands.  The reference runs this per frame on the
 // host ("always start from the depth seen by the RGB camera",
 // z_yooji_object_scanner.cpp:806-820).  Here one thread per depth pixel
-// lands its depth with an atomic minimum on the value's bits, which orders
+// lands its depth by compare-and-swap on the value's bits, which order
 // positive floats (and uint16) as their values, so the result does not
 // depend on the order the threads arrive in.
+//
+// The minimum runs in the caller's output itself, where 0 is both "empty" and
+// the answer for a pixel where nothing lands: two small launches, and the
+// host's part of them, bound it (512x424 into 1280x960: 20 us a call).  With a
+// scratch image from the stream's pool, a minimum beside "all ones" and a pass
+// to the output, 24 to 27 us, and 300 us when the pool had given its memory
+// back to the system between two calls.  Only an output that overlaps the
+// input needs the scratch.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -30,10 +38,31 @@ struct WarpArgs {
   float scale;  // depth units -> metres (1 for metres)
 };
 
-// T: depth type (float metres or uint16 units); out holds the minimum as
-// unsigned bits, "empty" = all ones
+// T is float (metres) or uint16 (units); the bits that order a depth
+__device__ __forceinline__ unsigned order_bits(float, float td) { return __float_as_uint(td); }
+__device__ __forceinline__ unsigned short order_bits(uint16_t raw, float) { return raw; }
+
+// the smallest of the values that land on *p, 0: none yet
+template <class W>
+__device__ __forceinline__ void land(W* p, W v) {
+  W old = *(volatile W*)p;
+  while (old == 0 || v < old) {  // after the first value, the stored one falls at each turn
+    const W seen = atomicCAS(p, old, v);
+    if (seen == old) break;
+    old = seen;
+  }
+}
 template <class T>
-__global__ void k_warp_depth(const T* __restrict__ in, WarpArgs a, unsigned* __restrict__ out) {
+struct Bits {
+  typedef unsigned word;
+};
+template <>
+struct Bits<uint16_t> {
+  typedef unsigned short word;
+};
+
+template <class T>
+__global__ void k_warp_depth(const T* __restrict__ in, WarpArgs a, typename Bits<T>::word* __restrict__ out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
   if (i >= a.wd || j >= a.hd) return;
   const T raw = in[(size_t)j * a.wd + i];
@@ -45,30 +74,27 @@ __global__ void k_warp_depth(const T* __restrict__ in, WarpArgs a, unsigned* __r
   if (isnan(u) || isnan(v)) return;
   const int tx = roundf_ref(u), ty = roundf_ref(v);
   if (tx < 0 || tx > a.wr - 1 || ty < 0 || ty > a.hr - 1) return;
-  unsigned bits;
-  if (sizeof(T) == 4)
-    bits = __float_as_uint(td);
-  else
-    bits = (unsigned)raw;
-  atomicMin(out + (size_t)ty * a.wr + tx, bits);
+  land(out + (size_t)ty * a.wr + tx, order_bits(raw, td));
 }
 
-template <class T>
-__global__ void k_warp_finish(const unsigned* __restrict__ bits, T* __restrict__ out, int n) {
+// zeroes n values: the 16-byte words among them, and the values before and
+// after those
+template <class W>
+__global__ void k_warp_clear(W* p, int n) {
+  constexpr int E = 16 / sizeof(W);
+  const int head = min(n, (int)((16 - (reinterpret_cast<uintptr_t>(p) & 15)) & 15) / (int)sizeof(W));
+  const int body = (n - head) / E, tail = n - head - body * E;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const unsigned b = bits[i];
-  if (sizeof(T) == 4)
-    reinterpret_cast<unsigned*>(out)[i] = (b == 0xffffffffu) ? 0u : b;
-  else
-    out[i] = (T)((b == 0xffffffffu) ? 0u : b);
+  if (i < body) reinterpret_cast<uint4*>(p + head)[i] = make_uint4(0u, 0u, 0u, 0u);
+  if (i < head) p[i] = 0;
+  if (i < tail) p[n - 1 - i] = 0;
 }
 
 }  // namespace
 
 template <class T>
 void launch_warp_depth(const T* in, int wd, int hd, const float* Kd, const float* T_rgb_d, const float* Kr, int wr,
-                       int hr, float scale, unsigned* scratch, T* out, cudaStream_t st) {
+                       int hr, float scale, T* out, cudaStream_t st) {
   WarpArgs a;
   a.wd = wd;
   a.hd = hd;
@@ -78,14 +104,16 @@ void launch_warp_depth(const T* in, int wd, int hd, const float* Kd, const float
   for (int k = 0; k < 12; k++) a.T[k] = T_rgb_d[k];
   a.scale = scale;
   const int n = wr * hr;
-  cudaMemsetAsync(scratch, 0xff, (size_t)n * 4, st);
-  k_warp_depth<T><<<dim3((wd + 31) / 32, (hd + 7) / 8), dim3(32, 8), 0, st>>>(in, a, scratch);
-  k_warp_finish<T><<<(n + 255) / 256, 256, 0, st>>>(scratch, out, n);
+  typedef typename Bits<T>::word W;
+  W* bits = reinterpret_cast<W*>(out);
+  const int blocks = (n / (16 / (int)sizeof(W)) + 16 + 255) / 256;
+  k_warp_clear<W><<<blocks, 256, 0, st>>>(bits, n);
+  k_warp_depth<T><<<dim3((wd + 31) / 32, (hd + 7) / 8), dim3(32, 8), 0, st>>>(in, a, bits);
 }
 
 template void launch_warp_depth<float>(const float*, int, int, const float*, const float*, const float*, int, int,
-                                       float, unsigned*, float*, cudaStream_t);
+                                       float, float*, cudaStream_t);
 template void launch_warp_depth<uint16_t>(const uint16_t*, int, int, const float*, const float*, const float*, int,
-                                          int, float, unsigned*, uint16_t*, cudaStream_t);
+                                          int, float, uint16_t*, cudaStream_t);
 
 }  // namespace vs

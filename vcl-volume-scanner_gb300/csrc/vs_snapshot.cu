@@ -39,7 +39,7 @@ void launch_bricks_copy(const SessionDev& h, const uint32_t* bricks, int n, void
                         bool to_packed, cudaStream_t st);
 template <class T>
 void launch_warp_depth(const T* in, int wd, int hd, const float* Kd, const float* T_rgb_d, const float* Kr, int wr,
-                       int hr, float scale, unsigned* scratch, T* out, cudaStream_t st);
+                       int hr, float scale, T* out, cudaStream_t st);
 }  // namespace vs
 
 using namespace vs;
@@ -318,14 +318,22 @@ static int warp_checks(const void* in, int wd, int hd, const float* Kd, const fl
 template <class T>
 static int warp_run(const T* in, int wd, int hd, const float* Kd, const float* Tm, const float* Kr, int wr, int hr,
                     float scale, T* out, void* stream) {
-  unsigned* scratch = nullptr;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(&scratch), (size_t)wr * hr * 4, st);
+  const size_t bytes = (size_t)wr * hr * sizeof(T);
+  const uintptr_t i0 = reinterpret_cast<uintptr_t>(in), o0 = reinterpret_cast<uintptr_t>(out);
+  // an output that shares memory with the input is formed beside it
+  const bool apart = o0 + bytes <= i0 || i0 + (size_t)wd * hd * sizeof(T) <= o0;
+  T* dst = out;
+  cudaError_t e = cudaSuccess;
+  if (!apart) e = cudaMallocAsync(reinterpret_cast<void**>(&dst), bytes, st);
   if (e != cudaSuccess) return cuda_fail_code(e, "warp scratch");
-  launch_warp_depth<T>(in, wd, hd, Kd, Tm, Kr, wr, hr, scale, scratch, out, st);
+  launch_warp_depth<T>(in, wd, hd, Kd, Tm, Kr, wr, hr, scale, dst, st);
   e = cudaGetLastError();
-  cudaError_t e2 = cudaFreeAsync(scratch, st);
-  if (e == cudaSuccess) e = e2;
+  if (!apart) {
+    if (e == cudaSuccess) e = cudaMemcpyAsync(out, dst, bytes, cudaMemcpyDeviceToDevice, st);
+    const cudaError_t e2 = cudaFreeAsync(dst, st);
+    if (e == cudaSuccess) e = e2;
+  }
   if (e != cudaSuccess) return cuda_fail_code(e, "depth warp");
   return VS_OK;
 }
