@@ -45,43 +45,60 @@ __device__ float g_inv_weight[65536];
 // when kept, the per-pixel ray scale lambda^-1 = 1 / |K^-1 [x y 1]| of
 // g_ctvc (z_yooji_cuda_volume_integrator.cu:357-372), each with the
 // reference's own operations
-__global__ void k_session_tables(SessionDev* s) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int d0 = s->dim[0], d1 = s->dim[1], d2 = s->dim[2];
-  if (i < d0) s->lut_vox[i] = ((float)i + 0.5f) / s->vox_inv + s->origin[0];
-  if (i < d1) s->lut_vox[d0 + i] = ((float)i + 0.5f) / s->vox_inv + s->origin[1];
-  if (i < d2) s->lut_vox[d0 + d1 + i] = ((float)i + 0.5f) / s->vox_inv + s->origin[2];
-  const float* K = s->lv[0].K;
-  const int W = s->lv[0].W, H = s->lv[0].H;
-  if (i < W) s->lut_ray[i] = 1.0f * ((float)i - K[2]) / K[0];
-  if (i < H) s->lut_ray[W + i] = 1.0f * ((float)i - K[3]) / K[1];
+__device__ __forceinline__ void session_tables(const SessionDev& s, int i) {
+  const int d0 = s.dim[0], d1 = s.dim[1], d2 = s.dim[2];
+  if (i < d0) s.lut_vox[i] = ((float)i + 0.5f) / s.vox_inv + s.origin[0];
+  if (i < d1) s.lut_vox[d0 + i] = ((float)i + 0.5f) / s.vox_inv + s.origin[1];
+  if (i < d2) s.lut_vox[d0 + d1 + i] = ((float)i + 0.5f) / s.vox_inv + s.origin[2];
+  const float* K = s.lv[0].K;
+  const int W = s.lv[0].W, H = s.lv[0].H;
+  if (i < W) s.lut_ray[i] = 1.0f * ((float)i - K[2]) / K[0];
+  if (i < H) s.lut_ray[W + i] = 1.0f * ((float)i - K[3]) / K[1];
   if (i < 65536) g_inv_weight[i] = 1.0f / (float)i;
-  if (s->lam_map && i < W * H) {
+  if (s.lam_map && i < W * H) {
     const int x = i % W, y = i / W;
     const float rx = 1.0f * ((float)x - K[2]) / K[0], ry = 1.0f * ((float)y - K[3]) / K[1];
-    s->lam_map[i] = 1.0f / sqrtf(rx * rx + ry * ry + 1.0f);
+    s.lam_map[i] = 1.0f / sqrtf(rx * rx + ry * ry + 1.0f);
   }
+}
+__global__ void k_session_tables(const SessionDev* __restrict__ s) {
+  session_tables(*s, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
-// frame counters of every slot, and the activation stamp.  A brick's flag
-// holds the stamp of the last integration that activated it, so no pass
-// clears flags: the flagged set of the last integration is {b : flag[b] ==
-// stamp != 0}, the reference's per-sub-cube bytes (cube_valid) after its
-// reset and marking (z_yooji_cuda_volume_integrator.cu:1006-1016), which
-// g_uvv_Update_Valid_Volume visits later.  A session whose tracking failed
-// (gate) does not integrate and keeps its stamp and flags.
-__global__ void k_integrate_prepare(const BatchTable* __restrict__ bt, int gate) {
-  const int i = threadIdx.x;
-  if (i < bt->n) {
-    const SessionDev* s = bt->s[i];
-    s->brick_count[0] = 0u;
-    s->brick_count[1] = 0u;
-    if (!(gate && s->pose->failed)) {
-      const uint32_t stamp = s->brick_count[2] + 1u;
-      s->brick_count[2] = stamp ? stamp : 1u;
-    }
-  }
+// The set-up of a call that brings its own volume: the descriptor and the
+// one-slot work table (kernel arguments) into their scratch, its tables, and
+// its counters and activation flags cleared
+__global__ void k_call_setup(const __grid_constant__ SessionDev h, const __grid_constant__ BatchTable t, SessionDev* d,
+                             BatchTable* dt, uint32_t nbr) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  constexpr uint32_t kHw = sizeof(SessionDev) / 4, kTw = sizeof(BatchTable) / 4;
+  static_assert(sizeof(SessionDev) % 4 == 0 && sizeof(BatchTable) % 4 == 0, "word copies");
+  static_assert(sizeof(SessionDev) + sizeof(BatchTable) + 64 <= 32764, "arguments exceed the parameter space");
+  if (i < kHw) reinterpret_cast<uint32_t*>(d)[i] = reinterpret_cast<const uint32_t*>(&h)[i];
+  if (i < kTw) reinterpret_cast<uint32_t*>(dt)[i] = reinterpret_cast<const uint32_t*>(&t)[i];
+  if (i < kBrickCounters) h.brick_count[i] = 0u;
+  for (uint32_t k = i; k < nbr; k += gridDim.x * blockDim.x) h.brick_flag[k] = 0u;
+  session_tables(h, (int)i);
 }
+
+// The counters of a session (brick_count), handed from one integration's two
+// kernels to the next integration's, so that no launch stands between them to
+// clear them:
+//   [0] active bricks, [1] voxels updated, of the last integration
+//   [2] activation stamp of the last integration (0: none yet)
+//   [3] which of the two list counters, [4] or [5], the next one counts in
+//   [6] what activation found: that choice, or kNoUpdate; [7] its new stamp
+// Activation reads [2] and [3], counts in [4] or [5], and writes [1], [6] and
+// [7]; the update reads [4] to [7], and writes [0], [2], [3] and, for the next
+// time, the other list counter.  A session whose tracking failed (gate) does
+// not integrate and keeps its stamp and flags.
+//
+// A brick's flag holds the stamp of the last integration that activated it, so
+// no pass clears flags: the flagged set of the last integration is {b :
+// flag[b] == stamp != 0}, the reference's per-sub-cube bytes (cube_valid)
+// after its reset and marking (z_yooji_cuda_volume_integrator.cu:1006-1016),
+// which g_uvv_Update_Valid_Volume visits later.
+constexpr uint32_t kNoUpdate = 2u;
 
 // What activation needs of a session, in shared memory: a block's rows nearly
 // all belong to one session.
@@ -101,7 +118,7 @@ struct __align__(16) ActSession {
 };
 
 __device__ inline void load_session(ActSession& a, const SessionDev* __restrict__ s, const float* depth_ext,
-                                    const float* Tcg_ext, bool gate, bool dry) {
+                                    const float* Tcg_ext, bool gate, bool dry, bool first) {
   const float* __restrict__ T = Tcg_ext ? Tcg_ext : s->pose->Tcg;
 #pragma unroll
   for (int k = 0; k < 3; k++) a.T[k] = make_float4(T[4 * k], T[4 * k + 1], T[4 * k + 2], T[4 * k + 3]);
@@ -110,7 +127,9 @@ __device__ inline void load_session(ActSession& a, const SessionDev* __restrict_
   a.grid = make_float4(s->origin[0], s->origin[1], s->origin[2], s->vox_inv);
   a.edge = make_float4((float)s->dim[0] - 0.5f, (float)s->dim[1] - 0.5f, (float)s->dim[2] - 0.5f, s->mu);
   for (int k = 0; k < 3; k++) a.nb[k] = s->nb[k];
-  a.stamp = s->brick_count[2];
+  a.stamp = s->brick_count[2] + 1u;
+  if (a.stamp == 0u) a.stamp = 1u;
+  const uint32_t turn = s->brick_count[3];
   a.W = s->lv[0].W;
   a.H = s->lv[0].H;
   a.tw = (a.W + 31) / 32;
@@ -118,8 +137,13 @@ __device__ inline void load_session(ActSession& a, const SessionDev* __restrict_
   a.depth = depth_ext ? depth_ext : s->depth_raw;
   a.flags = s->brick_flag;
   a.list = s->brick_list;
-  a.count = s->brick_count;
+  a.count = s->brick_count + 4 + turn;
   a.band = dry ? nullptr : s->band;
+  if (first) {
+    s->brick_count[1] = 0u;
+    s->brick_count[6] = a.skip ? kNoUpdate : turn;
+    s->brick_count[7] = a.stamp;
+  }
 }
 
 __device__ __forceinline__ F3 transform(F3 p, const float4 (&T)[3]) {
@@ -157,7 +181,9 @@ __global__ void __launch_bounds__(256, kActBlocks) k_activate(const BatchTable* 
       while (item >= next);
       base = bt->bil[slot];
       __syncthreads();
-      if (threadIdx.x == 0 && threadIdx.y == 0) load_session(a, bt->s[slot], depth_ext, Tcg_ext, gate != 0, dry != 0);
+      // the block of the session's first tile passes on what the update needs
+      if (threadIdx.x == 0 && threadIdx.y == 0)
+        load_session(a, bt->s[slot], depth_ext, Tcg_ext, gate != 0, dry != 0, item == base);
       __syncthreads();
     }
     if (a.skip) {
@@ -516,8 +542,22 @@ __global__ void __launch_bounds__(kIntThreads, COLOR ? kIntColorBlocks : kIntBlo
   const int n = bt->n;
   if (threadIdx.x < 32) {
     const int ln = threadIdx.x;
-    const uint32_t c0 = (2 * ln < n) ? *((volatile uint32_t*)bt->s[2 * ln]->brick_count) : 0u;
-    const uint32_t c1 = (2 * ln + 1 < n) ? *((volatile uint32_t*)bt->s[2 * ln + 1]->brick_count) : 0u;
+    auto listed = [&](int i) -> uint32_t {
+      if (i >= n) return 0u;
+      uint32_t* bc = bt->s[i]->brick_count;
+      const uint4 c = __ldcg(reinterpret_cast<const uint4*>(bc) + 1);  // [4] to [7]
+      const uint32_t count = c.z == kNoUpdate ? 0u : c.z ? c.y : c.x;
+      if (blockIdx.x == 0) {  // nothing in this launch reads these
+        bc[0] = count;
+        if (c.z != kNoUpdate) {
+          bc[2] = c.w;
+          bc[3] = c.z ^ 1u;
+          bc[4 + (c.z ^ 1u)] = 0u;
+        }
+      }
+      return count;
+    };
+    const uint32_t c0 = listed(2 * ln), c1 = listed(2 * ln + 1);
     uint32_t v = c0 + c1;
 #pragma unroll
     for (int m = 1; m < 32; m <<= 1) {
@@ -873,10 +913,14 @@ void launch_session_tables(const SessionDev& h, SessionDev* d, cudaStream_t st) 
   k_session_tables<<<(m + 255) / 256, 256, 0, st>>>(d);
 }
 
+void launch_call_setup(const SessionDev& h, const BatchTable& t, SessionDev* d, BatchTable* dt, cudaStream_t st) {
+  const int nbr = h.nb[0] * h.nb[1] * h.nb[2];
+  k_call_setup<<<256, 256, 0, st>>>(h, t, d, dt, (uint32_t)nbr);  // 65,536 threads: the weight table's entries
+}
+
 void launch_integrate(const BatchTable* bt, int tsdf_type, const float* depth, const float* Tgc, const float* Tcg,
                       bool gate, cudaStream_t st, bool color, int blocks_per_sm, bool dry) {
   const int c = color ? 1 : 0;
-  k_integrate_prepare<<<1, kMaxSlots, 0, st>>>(bt, gate ? 1 : 0);
   k_activate<<<sm_count() * kActBlocks, dim3(32, 8), 0, st>>>(bt, depth, Tcg, gate ? 1 : 0, dry ? 1 : 0);
   // persistent grid: every block resident at once
   switch (tsdf_type) {

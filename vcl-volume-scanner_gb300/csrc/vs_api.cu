@@ -149,7 +149,7 @@ int reset_state(vs_session* s) {
   VS_CU(cudaGetLastError());
   VS_CU(cudaMemsetAsync(s->h.brick_flag, 0, sizeof(uint32_t) * (size_t)s->h.nb[0] * s->h.nb[1] * s->h.nb[2],
                         s->stream));
-  VS_CU(cudaMemsetAsync(s->h.brick_count, 0, 4 * sizeof(uint32_t), s->stream));
+  VS_CU(cudaMemsetAsync(s->h.brick_count, 0, kBrickCounters * sizeof(uint32_t), s->stream));
   launch_occupancy_clear(s->h, s->stream);
   VS_CU(cudaGetLastError());
   VS_CU(cudaMemsetAsync(s->h.icp_counter, 0, sizeof(unsigned), s->stream));
@@ -877,7 +877,7 @@ int vs_kernels_per_frame(const vs_config* c) {
   int n = 1 + (kMaxLevels - 1);             // bilateral + pyramid levels
   if (c->cos_normal > -2.0f) n += 3;        // input maps: pre, row scan, post
   n += 2;                                   // ICP begin, every iteration
-  n += 3;                                   // counter reset, activation, update
+  n += 2;                                   // activation, update
   n += 2 + (c->color ? 2 : 1);              // band distances; ray march and shading of every level
   return n;
 }

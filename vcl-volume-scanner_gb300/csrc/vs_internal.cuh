@@ -19,6 +19,7 @@ constexpr int kBrick = 8;             // 8^3 voxels per brick = reference sub-cu
 constexpr int kBrickVox = 512;
 constexpr float kQ = 32767.0f;
 constexpr int kPartials = 32;         // partial slots per ICP block (29 used)
+constexpr int kBrickCounters = 8;
 constexpr int kIcpMaxBlocks = 456;    // 3 blocks per SM on 152 SMs
 constexpr int kMaxSlots = 64;         // sessions per batched launch
 
@@ -81,7 +82,8 @@ struct SessionDev {
   void* vol;                     // bricks, 512 words each
   uint32_t* brick_flag;          // per brick: stamp of the last integration that listed it (0: never / carved)
   uint32_t* brick_list;          // active bricks of this frame
-  uint32_t* brick_count;         // [0] active bricks, [1] voxels updated (per frame), [2] activation stamp
+  uint32_t* brick_count;         // [kBrickCounters]: [0] active bricks, [1] voxels updated (of the last integration),
+                                 // [2] activation stamp, [3..7] between the two kernels (k_integrate.cu)
   uint32_t* occ;                 // 1 bit per brick: some voxel has weight > 0 (NULL: not kept)
   uint8_t* band;                 // per brick: 1 if some voxel has weight > 0 and a TSDF value other
                                  // than 1 (a superset is allowed; NULL: not kept)
