@@ -271,7 +271,7 @@ size_t vs_session_bytes(const vs_config* c) {
   if (check_config(c) != VS_OK) return 0;
   size_t b = volume_bytes(c);
   size_t nbr = (size_t)(c->dim[0] / 8) * (c->dim[1] / 8) * (c->dim[2] / 8);
-  b += 2 * nbr * 4 + ((nbr + 31) / 32) * 4 + 3 * nbr + 64;
+  b += 2 * nbr * 4 + ((nbr + 31) / 32) * 4 + 2 * nbr + 64;
   int w = c->width, h = c->height;
   b += (size_t)w * h * (2 + 4 + 4);
   for (int l = 0; l < c->levels; l++) {
@@ -326,7 +326,6 @@ int vs_session_create(const vs_config* cfg, vs_session** out) {
   rc |= alloc(s, &h.occ, occupancy_words(h) * 4);
   rc |= alloc(s, &h.band, nbr);
   rc |= alloc(s, &h.bdist, nbr);
-  rc |= alloc(s, &h.btmp, nbr);
   rc |= alloc(s, &h.depth_mm, n0 * 2);
   rc |= alloc(s, &h.depth_raw, n0 * 4);
   rc |= alloc(s, &s->stage_f, n0 * 4);
@@ -878,7 +877,7 @@ int vs_kernels_per_frame(const vs_config* c) {
   if (c->cos_normal > -2.0f) n += 3;        // input maps: pre, row scan, post
   n += 2;                                   // ICP begin, every iteration
   n += 2;                                   // activation, update
-  n += 2 + (c->color ? 2 : 1);              // band distances; ray march and shading of every level
+  n += 1 + (c->color ? 2 : 1);              // band distances; ray march and shading of every level
   return n;
 }
 

@@ -89,7 +89,6 @@ struct SessionDev {
                                  // than 1 (a superset is allowed; NULL: not kept)
   uint8_t* bdist;                // per brick: Chebyshev distance in bricks to the nearest band brick,
                                  // saturating at kBandReach + 1 (rebuilt before every ray-cast)
-  uint8_t* btmp;                 // the distance transform's intermediate (x and y passes)
   // ICP scratch
   double* partials;              // [kIcpMaxBlocks][2*kPartials]
   unsigned* icp_counter;
@@ -131,8 +130,7 @@ struct BatchTable {
   const uint16_t* frame[kMaxSlots];    // the uint16 frame each slot's ingest reads in place this step (device
                                        // memory, or pinned host memory the device can address; the ingest
                                        // also copies it into the session's frame buffer); NULL: that buffer
-  int slab[kMaxSlots + 1];             // z slabs of bricks (band distance, x and y passes)
-  int brow[kMaxSlots + 1];             // y rows of bricks (band distance, z pass)
+  int slab[kMaxSlots + 1];             // z slabs of bricks (band distance)
   unsigned work[8];                    // work counters ([0..1] ray march, [4..5] ray shading); zero between
                                        // launches
   unsigned icp_word[kMaxSlots];        // per slot: level, iteration and next range of its tracking (k_icp.cu)
