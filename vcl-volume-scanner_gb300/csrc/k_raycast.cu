@@ -38,7 +38,7 @@ struct RayArgs {
   // explicit poses and outputs of a one-level, one-slot call (reference layout)
   const float* Tgc;
   const float* Tcg;
-  const float* center;  // device float[3]
+  float center[3];
   float light[3];
   int gate;
   float* out_depth;
@@ -464,8 +464,8 @@ __device__ inline void load_tile_cam(const RayArgs& a, const SessionDev& s, int 
   const bool ext = a.level >= 0;
   const float* Tcg = ext ? a.Tcg : s.pose->Tcg;
   const float* Tgc = ext ? a.Tgc : s.pose->Tgc;
-  const float* cen = ext ? a.center : s.pose->center;
-  const F3 cam = f3(cen[0], cen[1], cen[2]);
+  const F3 cam = ext ? f3(a.center[0], a.center[1], a.center[2])
+                     : f3(s.pose->center[0], s.pose->center[1], s.pose->center[2]);
   // host-side set-up of rmi_Render_Maps_for_ICP (:1667-1675)
   const F3 cc = f3(s.cube_center[0], s.cube_center[1], s.cube_center[2]);
   const F3 vcc = sub(cc, cam);
@@ -910,7 +910,7 @@ void launch_raycast(const BatchTable* bt, int tsdf_type, int level, const float*
   a.level = level;
   a.Tgc = Tgc;
   a.Tcg = Tcg;
-  a.center = center;
+  for (int k = 0; k < 3; k++) a.center[k] = center ? center[k] : 0.0f;  // by value: no copy goes before the launch
   a.light[0] = lx;
   a.light[1] = ly;
   a.light[2] = lz;

@@ -484,8 +484,7 @@ int vs_render_maps(vs_session* s, int ww, int hh, const float* T_gc_dev, const f
     return fail(VS_ERR_ARG, "null argument");
   if (level < 0 || level >= s->h.levels) return fail(VS_ERR_ARG, "bad level");
   if (ww != s->h.lv[level].W || hh != s->h.lv[level].H) return fail(VS_ERR_ARG, "size differs from the level");
-  VS_CU(cudaMemcpyAsync(s->dev_small, cam_cen, 3 * sizeof(float), cudaMemcpyHostToDevice, s->stream));
-  launch_raycast(s->tab, s->h.tsdf_type, level, T_gc_dev, T_cg_dev, s->dev_small, light[0], light[1], light[2],
+  launch_raycast(s->tab, s->h.tsdf_type, level, T_gc_dev, T_cg_dev, cam_cen, light[0], light[1], light[2],
                  false, depth_dev, vtx_dev, nrm_dev, img_dev, s->stream);
   VS_CU(cudaGetLastError());
   VS_CU(cudaStreamSynchronize(s->stream));
@@ -500,8 +499,7 @@ int vs_render_maps_color(vs_session* s, int ww, int hh, const float* T_gc_dev, c
   if (!s->h.col) return fail(VS_ERR_STATE, "session has no colour volume (cfg.color = 0)");
   if (level < 0 || level >= s->h.levels) return fail(VS_ERR_ARG, "bad level");
   if (ww != s->h.lv[level].W || hh != s->h.lv[level].H) return fail(VS_ERR_ARG, "size differs from the level");
-  VS_CU(cudaMemcpyAsync(s->dev_small, cam_cen, 3 * sizeof(float), cudaMemcpyHostToDevice, s->stream));
-  launch_raycast(s->tab, s->h.tsdf_type, level, T_gc_dev, T_cg_dev, s->dev_small, light[0], light[1], light[2],
+  launch_raycast(s->tab, s->h.tsdf_type, level, T_gc_dev, T_cg_dev, cam_cen, light[0], light[1], light[2],
                  false, depth_dev, vtx_dev, nrm_dev, img_dev, s->stream, LaunchShape(), rgb_dev, true);
   VS_CU(cudaGetLastError());
   VS_CU(cudaStreamSynchronize(s->stream));
@@ -517,8 +515,7 @@ static int render_variant(vs_session* s, int ww, int hh, const float* T_gc_dev, 
   if (rgb_dev && !s->h.col) return fail(VS_ERR_STATE, "session has no colour volume (cfg.color = 0)");
   if (level < 0 || level >= s->h.levels) return fail(VS_ERR_ARG, "bad level");
   if (ww != s->h.lv[level].W || hh != s->h.lv[level].H) return fail(VS_ERR_ARG, "size differs from the level");
-  VS_CU(cudaMemcpyAsync(s->dev_small, cam_cen, 3 * sizeof(float), cudaMemcpyHostToDevice, s->stream));
-  launch_raycast(s->tab, s->h.tsdf_type, level, T_gc_dev, T_cg_dev, s->dev_small, light[0], light[1], light[2],
+  launch_raycast(s->tab, s->h.tsdf_type, level, T_gc_dev, T_cg_dev, cam_cen, light[0], light[1], light[2],
                  false, depth_dev, vtx_dev, nrm_dev, img_dev, s->stream, LaunchShape(), rgb_dev, rgb_dev != nullptr,
                  mode);
   VS_CU(cudaGetLastError());

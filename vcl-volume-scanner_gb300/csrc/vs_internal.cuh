@@ -335,7 +335,8 @@ void launch_integrate(const BatchTable* bt, int tsdf_type, const float* depth, c
                       const float* Tcg, bool gate_on_tracking, cudaStream_t st, bool color = false,
                       int blocks_per_sm = 0, bool dry = false);
 // level < 0: every level of every slot into the sessions' model maps; else
-// one level of a one-slot table into the external outputs with explicit poses;
+// one level of a one-slot table into the external outputs with explicit poses
+// (center: on the host);
 // color: the shading variant that also interpolates colour
 void launch_raycast(const BatchTable* bt, int tsdf_type, int level, const float* Tgc, const float* Tcg,
                     const float* center, float lx, float ly, float lz, bool gate_on_tracking, float* out_depth,
