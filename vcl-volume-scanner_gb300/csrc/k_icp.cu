@@ -115,6 +115,55 @@ __device__ inline bool icp_term(int x, int y, int w, int h, const float* K, floa
   return true;
 }
 
+// Two pixels with the normal test at once: the same operations without a
+// branch, so that the taps of both are in flight together
+__device__ __forceinline__ void icp_pair(const int (&x)[2], const int (&y)[2], int w, int h, const float* K,
+                                         const float (&d1)[2], const float4 (&q)[2], const float4* __restrict__ mvtx,
+                                         const float4* __restrict__ mnrm, const float* T21, float th_icp,
+                                         float cos_normal, float (&A)[2][6], float (&b)[2], bool (&ok)[2]) {
+  F3 p0[2], p1[2];
+  Taps t[2];
+  float4 v[2][4];
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    p1[k] = transform(back_project((float)x[k], (float)y[k], K, d1[k]), T21);
+    float u, vv;
+    project(p1[k], K, u, vv);
+    ok[k] = tap_setup(u, vv, w, h, t[k]) && !(d1[k] < 1.0e-6f);
+    if (!ok[k]) t[k].i00 = t[k].i01 = t[k].i10 = t[k].i11 = 0, t[k].rx = t[k].ry = 0.0f;  // (the map's first value)
+  }
+#pragma unroll
+  for (int k = 0; k < 2; k++)
+    v[k][0] = __ldg(mvtx + t[k].i00), v[k][1] = __ldg(mvtx + t[k].i01), v[k][2] = __ldg(mvtx + t[k].i10),
+    v[k][3] = __ldg(mvtx + t[k].i11);
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    ok[k] &= interp(t[k], v[k][0], v[k][1], v[k][2], v[k][3], p0[k]);
+    const float dd = (p0[k].x - p1[k].x) * (p0[k].x - p1[k].x) + (p0[k].y - p1[k].y) * (p0[k].y - p1[k].y) +
+                     (p0[k].z - p1[k].z) * (p0[k].z - p1[k].z);
+    ok[k] &= !(dd > th_icp);
+  }
+#pragma unroll
+  for (int k = 0; k < 2; k++)
+    v[k][0] = __ldg(mnrm + t[k].i00), v[k][1] = __ldg(mnrm + t[k].i01), v[k][2] = __ldg(mnrm + t[k].i10),
+    v[k][3] = __ldg(mnrm + t[k].i11);
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    F3 n;
+    ok[k] &= interp(t[k], v[k][0], v[k][1], v[k][2], v[k][3], n);
+    n = normalised(n);
+    const F3 nin = rotate(f3(q[k].x, q[k].y, q[k].z), T21);
+    ok[k] &= q[k].w != 0.0f && !(dot(nin, n) < cos_normal);
+    A[k][0] = p1[k].z * n.y + (-p1[k].y) * n.z;
+    A[k][1] = (-p1[k].z) * n.x + p1[k].x * n.z;
+    A[k][2] = p1[k].y * n.x + (-p1[k].x) * n.y;
+    A[k][3] = -n.x;
+    A[k][4] = -n.y;
+    A[k][5] = -n.z;
+    b[k] = dot(n, sub(p0[k], p1[k]));
+  }
+}
+
 // error-free addition (Knuth two-sum): s + e == a + b exactly
 __device__ inline void two_sum(float a, float b, float& s, float& e) {
   s = a + b;
@@ -251,6 +300,19 @@ __device__ inline double2 shfl_xor2(double2 v, int m) {
 }
 
 __device__ inline int tri_index(int i, int j) { return i * 6 - i * (i - 1) / 2 + (j - i); }
+
+// one pixel's products
+template <class ACC>
+__device__ __forceinline__ void add_term(ACC& acc, const float (&A)[6], float b) {
+#pragma unroll
+  for (int i = 0; i < 6; i++)
+#pragma unroll
+    for (int j = i; j < 6; j++) acc.add(tri_index(i, j), A[i] * A[j]);
+#pragma unroll
+  for (int i = 0; i < 6; i++) acc.add(21 + i, A[i] * b);
+  acc.add(27, 1.0f);
+  acc.add(28, b * b);
+}
 
 // ---- FP64 pose algebra ------------------------------------------------------
 // FP64 runs on a narrow pipe on this part: an operation of a warp takes 64
@@ -854,52 +916,74 @@ __global__ void __launch_bounds__(kThreads, VS_ICP_MIN_BLOCKS)
     // in flight while its current pixel's taps are read, and the list entry
     // of the one after that
     int p = vb * kThreads + threadIdx.x;
-    int x = 0, y = 0, dx = 0, dy = 0;
-    uint32_t xy = 0u;
-    float d_next = 0.0f;
-    float4 q_next = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    if (ntest) {
-      if (p < count) {
-        xy = __ldg(list + p);
-        x = (int)(xy & 0xffffu), y = (int)(xy >> 16);
-        d_next = __ldg(depth + y * w + x);
-        q_next = __ldg(innrm + y * w + x);
-        if (p + stride < count) xy = __ldg(list + p + stride);
+    if (MODE == VS_REDUCE_FP64 && ntest && count <= 2 * stride) {
+      // A listed range, at most two pixels per thread.  With FP64 sums, whose
+      // 58 registers leave the loop below no room to read ahead, the two are
+      // taken together before any sum is held (tracking of a 640x480 frame 332
+      // -> 315 us, sixteen sessions 1655 -> 1619); the float sums gain nothing
+      // (640x480 frames 385 and 385 us, a served mix 1050 and 1058).
+      int xs[2], ys[2];
+      float ds[2];
+      float4 qs[2];
+#pragma unroll
+      for (int k = 0; k < 2; k++) {
+        const uint32_t e = p + k * stride < count ? __ldg(list + p + k * stride) : 0u;
+        xs[k] = (int)(e & 0xffffu), ys[k] = (int)(e >> 16);
       }
+#pragma unroll
+      for (int k = 0; k < 2; k++) {
+        const bool in = p + k * stride < count;
+        ds[k] = in ? __ldg(depth + ys[k] * w + xs[k]) : 0.0f;
+        qs[k] = in ? __ldg(innrm + ys[k] * w + xs[k]) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      }
+      __syncthreads();  // the pose
+      float A[2][6], b[2];
+      bool ok[2];
+      icp_pair(xs, ys, w, h, K, ds, qs, mvtx, mnrm, T21, th, cosn, A, b, ok);
+#pragma unroll
+      for (int k = 0; k < 2; k++)
+        if (ok[k]) add_term(acc, A[k], b[k]);
     } else {
-      y = p / w, x = p - y * w;
-      dy = stride / w, dx = stride - dy * w;
-      if (p < count) d_next = __ldg(depth + p);
-    }
-    __syncthreads();
-    while (p < count) {
-      const float d1 = d_next;
-      const float4 qn = q_next;
-      const int xc = x, yc = y;
-      p += stride;
+      int x = 0, y = 0, dx = 0, dy = 0;
+      uint32_t xy = 0u;
+      float d_next = 0.0f;
+      float4 q_next = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
       if (ntest) {
         if (p < count) {
+          xy = __ldg(list + p);
           x = (int)(xy & 0xffffu), y = (int)(xy >> 16);
           d_next = __ldg(depth + y * w + x);
           q_next = __ldg(innrm + y * w + x);
           if (p + stride < count) xy = __ldg(list + p + stride);
         }
       } else {
-        x += dx;
-        y += dy;
-        if (x >= w) x -= w, y++;
+        y = p / w, x = p - y * w;
+        dy = stride / w, dx = stride - dy * w;
         if (p < count) d_next = __ldg(depth + p);
       }
-      float A[6], b;
-      if (!icp_term(xc, yc, w, h, K, d1, qn, mvtx, mnrm, T21, th, cosn, A, b)) continue;
-#pragma unroll
-      for (int i = 0; i < 6; i++)
-#pragma unroll
-        for (int j = i; j < 6; j++) acc.add(tri_index(i, j), A[i] * A[j]);
-#pragma unroll
-      for (int i = 0; i < 6; i++) acc.add(21 + i, A[i] * b);
-      acc.add(27, 1.0f);
-      acc.add(28, b * b);
+      __syncthreads();
+      while (p < count) {
+        const float d1 = d_next;
+        const float4 qn = q_next;
+        const int xc = x, yc = y;
+        p += stride;
+        if (ntest) {
+          if (p < count) {
+            x = (int)(xy & 0xffffu), y = (int)(xy >> 16);
+            d_next = __ldg(depth + y * w + x);
+            q_next = __ldg(innrm + y * w + x);
+            if (p + stride < count) xy = __ldg(list + p + stride);
+          }
+        } else {
+          x += dx;
+          y += dy;
+          if (x >= w) x -= w, y++;
+          if (p < count) d_next = __ldg(depth + p);
+        }
+        float A[6], b;
+        if (!icp_term(xc, yc, w, h, K, d1, qn, mvtx, mnrm, T21, th, cosn, A, b)) continue;
+        add_term(acc, A, b);
+      }
     }
     const PT mine = acc.reduce_scatter(lane);
     if (lane < 29) wsum[warp][lane] = mine;
