@@ -1080,6 +1080,23 @@ int icp_blocks(int npix, int level) {
   return b;
 }
 
+// An SM divides its storage between L1 and shared memory when its first block
+// arrives and keeps the division while a block runs.  By default it suits the
+// 4 to 6 KB of this launch's blocks, which then hold their SMs for the whole of
+// the tracking: kernels of a batch's other branch that need more (the scan of
+// the input maps, the update's partial sums, the filter) found no SM and the
+// branches ran one after the other.  With 40 % of the storage as shared memory
+// they fit beside: steps of 8, 12, 16 and 24 sessions 850 -> 725, 1172 -> 1018,
+// 1302 -> 1172 and 1766 -> 1655 us; of 1 and 64 the same.  (15 and 25 % the same
+// within 1 %; 60 and 100 % leave L1 too little, 1.5 and 3 % more with one
+// session or 64 of them.)
+void configure_icp_kernels() {
+  constexpr int kShared = 40;
+  cudaFuncSetAttribute(k_icp_run<VS_REDUCE_FP32>, cudaFuncAttributePreferredSharedMemoryCarveout, kShared);
+  cudaFuncSetAttribute(k_icp_run<VS_REDUCE_KAHAN>, cudaFuncAttributePreferredSharedMemoryCarveout, kShared);
+  cudaFuncSetAttribute(k_icp_run<VS_REDUCE_FP64>, cudaFuncAttributePreferredSharedMemoryCarveout, kShared);
+}
+
 void launch_icp(const BatchTable* bt, int reduce_mode, cudaStream_t st, bool frame_mode, const float* init_T12) {
   // frame-level calls skip tracking on the first frame as so_Scan_Object does
   // (zz_flag_track, z_yooji_object_scanner.cpp:534,572-576); explicit

@@ -26,6 +26,7 @@ namespace vs {
 void launch_volume_slab(const SessionDev& h, bool do_export, int z0, int nz, float* tsdf, uint16_t* w,
                         cudaStream_t st);
 void configure_filter_kernels();
+void configure_icp_kernels();
 int integrate_max_dim();
 int integrate_max_image();
 }  // namespace vs
@@ -298,7 +299,10 @@ int vs_session_create(const vs_config* cfg, vs_session** out) {
   int ndev = 0;
   cudaError_t e = cudaGetDeviceCount(&ndev);
   if (e != cudaSuccess || ndev == 0) return fail(VS_ERR_CUDA, "no CUDA device available");
-  std::call_once(g_once, [] { configure_filter_kernels(); });
+  std::call_once(g_once, [] {
+    configure_filter_kernels();
+    configure_icp_kernels();
+  });
   vs_session* s = new vs_session;
   s->cfg = *cfg;
   cudaGetDevice(&s->device);
