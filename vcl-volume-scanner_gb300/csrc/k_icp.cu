@@ -842,14 +842,18 @@ __device__ __noinline__ void claim_range(unsigned* __restrict__ words, int n, co
 // on noisy depth), in 15 to 30 % of the 32-pixel words.  Reading depth and model
 // taps of every pixel, tracking took 2.01 ms of the 64-session step and 0.606
 // of sixteen sessions'; over the list 0.52 and 0.26 (a 640x480 frame 490 ->
-// 434 us).  512 pixels per range: 256 and 1024 made a 640x480 frame 422 and 462
-// us, the 64-session step 4712 and 4456 us against 4505.  Every session has
-// at least one range, which closes its iterations.
-#ifndef VS_ICP_LISTED_PER_RANGE
-#define VS_ICP_LISTED_PER_RANGE 512
-#endif
+// 434 us).  A range of 256 pixels is one per thread, and its blocks are done
+// sooner; 512 pay the reduction of a range half as often.  Up to 8192 listed
+// pixels (by the session's own count alone, so that its sums do not depend on
+// what shares the launch) a level does not fill the launch's blocks: 256 there
+// made a 640x480 frame 385 -> 377 us, a 320x240 frame 313 -> 299, FP64 tracking
+// of 640x480 316 -> 285, sixteen sessions 1344 -> 1331, and 64 sessions 3872 ->
+// 3897 (two runs of one side: 35 apart).  256 at every count took 64 sessions
+// 4.5 % longer.  Every session has at least one range, which closes its
+// iterations.
 __device__ __forceinline__ int listed_ranges(int count) {
-  const int r = (count + VS_ICP_LISTED_PER_RANGE - 1) / VS_ICP_LISTED_PER_RANGE;
+  const int per = count <= 8192 ? kThreads : 2 * kThreads;
+  const int r = (count + per - 1) / per;
   return min(max(r, 1), kIcpMaxBlocks);
 }
 
@@ -917,7 +921,7 @@ __global__ void __launch_bounds__(kThreads, VS_ICP_MIN_BLOCKS)
     // of the one after that
     int p = vb * kThreads + threadIdx.x;
     if (MODE == VS_REDUCE_FP64 && ntest && count <= 2 * stride) {
-      // A listed range, at most two pixels per thread.  With FP64 sums, whose
+      // A listed range, one or two pixels per thread.  With FP64 sums, whose
       // 58 registers leave the loop below no room to read ahead, the two are
       // taken together before any sum is held (tracking of a 640x480 frame 332
       // -> 315 us, sixteen sessions 1655 -> 1619); the float sums gain nothing
