@@ -19,7 +19,7 @@ namespace vs {
 namespace {
 
 constexpr int BX = 32, BY = 8;  // threads of a filter block (BY: default rows; 4 and 16 also built)
-constexpr int kPerThread = 2;   // outputs per thread, consecutive rows
+constexpr int kPerThread = 2;   // outputs per thread, consecutive rows (1 also built, for small float maps)
 constexpr int kScanSmem = 64 * 1024;  // staged normal-rejection bitmasks of one level
 
 // The reference reads a linear-filtered texture at integer coordinates, so
@@ -35,10 +35,10 @@ constexpr int kScanSmem = 64 * 1024;  // staged normal-rejection bitmasks of one
 // test per tap.  With one output per thread in 32 x 8 tiles 1920x1080 took
 // 33.5 us, and takes 25.2; four rows per thread 26 us, and 2 us more for one
 // 640x480 frame, whose tiles are few.
-template <int R>
+template <int R, int P>
 struct BilateralSmem {
-  float tex[kPerThread * R + 5][BX + 6];
-  float tap[kPerThread * R + 4][BX + 5];
+  float tex[P * R + 5][BX + 6];
+  float tap[P * R + 4][BX + 5];
 };
 
 // exp2 by the special-function unit (ex2.approx.ftz.f32)
@@ -48,12 +48,12 @@ __device__ __forceinline__ float exp2_approx(float x) {
   return r;
 }
 
-// The filter of kPerThread pixels, rows ty0 .. of column tx.  Every sum runs in
+// The filter of P pixels, rows ty0 .. of column tx.  Every sum runs in
 // the reference's order with its roundings.  A tap that is not above 0 is stored as
 // -infinity: as the centre it makes the sum infinite, elsewhere its weight is
 // 0 and their product not a number.
-template <int R>
-__device__ inline void bilateral_px(const BilateralSmem<R>& m, int tx, int ty0, bool finite, float out[kPerThread]) {
+template <int R, int P>
+__device__ inline void bilateral_px(const BilateralSmem<R, P>& m, int tx, int ty0, bool finite, float out[P]) {
   // The Gaussian of delta 4 (:275-286), exp(-x^2 / (2 * 4^2)).  The range
   // weight's exponent is -mod / (2 sigma_r^2), 2 sigma_r^2 = 2.0f * 0.1f *
   // 0.1f with sigma_r = 0.1 m (z_yooji_cuda_img_proc.cu:44,91), here the
@@ -66,19 +66,19 @@ __device__ inline void bilateral_px(const BilateralSmem<R>& m, int tx, int ty0, 
   constexpr float g1 = 0.96923321f, g2 = 0.88249689f;  // exp(-1 / 32), exp(-4 / 32) rounded to float
   constexpr float g[5] = {g2, g1, 1.0f, g1, g2};
   constexpr float kNegInvDenom = -1.0f / (2.0f * 0.1f * 0.1f), kLog2e = 1.44269504f;
-  float c[kPerThread], t[kPerThread], sum[kPerThread];
+  float c[P], t[P], sum[P];
 #pragma unroll
-  for (int r = 0; r < kPerThread; r++) {
+  for (int r = 0; r < P; r++) {
     c[r] = m.tap[ty0 + r + 2][tx + 2];
     t[r] = sum[r] = 0.0f;
   }
 #pragma unroll
-  for (int k = 0; k < kPerThread + 4; k++) {
+  for (int k = 0; k < P + 4; k++) {
     float a[5];
 #pragma unroll
     for (int j = 0; j < 5; j++) a[j] = m.tap[ty0 + k][tx + j];
 #pragma unroll
-    for (int r = 0; r < kPerThread; r++) {
+    for (int r = 0; r < P; r++) {
       const int i = k - r;
       if (i < 0 || i > 4) continue;
 #pragma unroll
@@ -96,7 +96,7 @@ __device__ inline void bilateral_px(const BilateralSmem<R>& m, int tx, int ty0, 
     }
   }
 #pragma unroll
-  for (int r = 0; r < kPerThread; r++) {
+  for (int r = 0; r < P; r++) {
     out[r] = t[r] / sum[r];
     if (!(t[r] >= 0.0f)) {
       bool hole = finite;  // finite inputs: only a hole gives this
@@ -107,13 +107,13 @@ __device__ inline void bilateral_px(const BilateralSmem<R>& m, int tx, int ty0, 
   }
 }
 
-// one BX x 2R output tile; the block's BX x R threads all take part (two barriers)
-template <bool FROM_MM, int R>
-__device__ inline void bilateral_tile(BilateralSmem<R>& m, const uint16_t* __restrict__ mm,
+// one BX x P R output tile; the block's BX x R threads all take part (two barriers)
+template <bool FROM_MM, int R, int P>
+__device__ inline void bilateral_tile(BilateralSmem<R, P>& m, const uint16_t* __restrict__ mm,
                                       const float* __restrict__ fin, float scale, float* __restrict__ raw_out,
                                       float* __restrict__ out, int W, int H, int x0, int y0,
                                       float2* __restrict__ dl_out = nullptr, const float* __restrict__ lam = nullptr) {
-  constexpr int TR = kPerThread * R;
+  constexpr int TR = P * R;
   const int tx = threadIdx.x, ty = threadIdx.y;
   // a warp per texel row: BX columns, then the five beyond
 #pragma unroll
@@ -147,16 +147,16 @@ __device__ inline void bilateral_tile(BilateralSmem<R>& m, const uint16_t* __res
     }
   }
   __syncthreads();
-  const int x = x0 + tx, yb = y0 + ty * kPerThread;
+  const int x = x0 + tx, yb = y0 + ty * P;
   if (x < W && yb < H) {
-    float f[kPerThread];
-    bilateral_px(m, tx, ty * kPerThread, FROM_MM, f);
+    float f[P];
+    bilateral_px(m, tx, ty * P, FROM_MM, f);
 #pragma unroll
-    for (int r = 0; r < kPerThread; r++) {
+    for (int r = 0; r < P; r++) {
       if (yb + r >= H) break;
       const size_t i = (size_t)(yb + r) * W + x;
       if (FROM_MM) {
-        const float raw = m.tex[ty * kPerThread + r + 3][tx + 3];
+        const float raw = m.tex[ty * P + r + 3][tx + 3];
         raw_out[i] = raw;
         if (dl_out) dl_out[i] = make_float2(raw, __ldg(lam + i));
       }
@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(BX* BY) k_ingest(const BatchTable* __restrict_
 
 template <int R>
 __global__ void __launch_bounds__(BX* R) k_bilateral_batch(const BatchTable* __restrict__ bt) {
-  __shared__ BilateralSmem<R> m;
+  __shared__ BilateralSmem<R, kPerThread> m;
   const int n = bt->n;
   const int total = bt->fil[n];
   for (int item = blockIdx.x; item < total; item += gridDim.x) {
@@ -205,8 +205,8 @@ __global__ void __launch_bounds__(BX* R) k_bilateral_batch(const BatchTable* __r
     const int W = s->lv[0].W, H = s->lv[0].H;
     const int tw = (W + BX - 1) / BX, tyy = t / tw;
     const int x0 = (t - tyy * tw) * BX, y0 = tyy * R * kPerThread;
-    bilateral_tile<true, R>(m, s->depth_mm, nullptr, s->depth_scale, s->depth_raw, s->depth[0], W, H, x0, y0,
-                            s->lam_map ? s->dl_map : nullptr, s->lam_map);
+    bilateral_tile<true, R, kPerThread>(m, s->depth_mm, nullptr, s->depth_scale, s->depth_raw, s->depth[0], W, H, x0,
+                                        y0, s->lam_map ? s->dl_map : nullptr, s->lam_map);
     if (s->rgb_packed) {
       // the colour frame as one word per pixel, for the integration's gathers
       const int x = x0 + threadIdx.x;
@@ -219,10 +219,11 @@ __global__ void __launch_bounds__(BX* R) k_bilateral_batch(const BatchTable* __r
   }
 }
 
+template <int P>
 __global__ void __launch_bounds__(BX* BY, 6)
     k_bilateral_float(const float* __restrict__ in, float* __restrict__ out, int W, int H) {
-  __shared__ BilateralSmem<BY> m;
-  bilateral_tile<false, BY>(m, nullptr, in, 1.0f, nullptr, out, W, H, blockIdx.x * BX, blockIdx.y * BY * kPerThread);
+  __shared__ BilateralSmem<BY, P> m;
+  bilateral_tile<false, BY, P>(m, nullptr, in, 1.0f, nullptr, out, W, H, blockIdx.x * BX, blockIdx.y * BY * P);
 }
 
 // level l -> l+1: separable [1 4 6 4 1] smoothing (borders 0, no validity
@@ -611,8 +612,16 @@ void launch_input_maps(const BatchTable* bt, cudaStream_t st) {
 
 void launch_bilateral_float(const SessionDev& h, const float* in, float* out, cudaStream_t st) {
   const int W = h.lv[0].W, H = h.lv[0].H;
-  dim3 blk(BX, BY), grd((W + BX - 1) / BX, (H + BY * kPerThread - 1) / (BY * kPerThread));
-  k_bilateral_float<<<grd, blk, 0, st>>>(in, out, W, H);
+  const int cols = (W + BX - 1) / BX, rows = (H + BY - 1) / BY;
+  // One row per thread while its tiles are all resident (six blocks per SM):
+  // a thread's chain is half as long, 2.4 instead of 3.3 us for 160x120, 4.4
+  // and 4.6 for 512x424 (848 tiles); beyond, two rows: 640x480 5.9 and 5.6 us,
+  // 1920x1080 26.9 and 24.3.
+  if (cols * rows <= sm_count() * 6)
+    k_bilateral_float<1><<<dim3(cols, rows), dim3(BX, BY), 0, st>>>(in, out, W, H);
+  else
+    k_bilateral_float<kPerThread>
+        <<<dim3(cols, (rows + kPerThread - 1) / kPerThread), dim3(BX, BY), 0, st>>>(in, out, W, H);
 }
 
 void configure_filter_kernels() {
