@@ -243,14 +243,13 @@ def traffic_per_unit(kernel_key, unit_key):
 
 def raycast_per_unit(key):
     """(per ray, per sub-cube) figure of the ray-cast stage's kernels from the
-    committed ncu summary: the march-and-shade kernel per ray, the two passes
-    of the band distance field per sub-cube; key "dram_bytes" or "warp_inst" """
+    committed ncu summary: the march-and-shade kernel per ray, the band
+    distance field per sub-cube; key "dram_bytes" or "warp_inst" """
     r = traffic_per_unit("k_ray_fused", key + "_per_ray")
-    bx = traffic_per_unit("k_band_xy", key + "_per_brick")
-    bz = traffic_per_unit("k_band_z", key + "_per_brick")
-    if r is None or bx is None or bz is None:
+    b = traffic_per_unit("k_band", key + "_per_brick")
+    if r is None or b is None:
         return None
-    return r, bx + bz
+    return r, b
 
 
 def level_bricks(cfg):
@@ -734,7 +733,7 @@ def run_ours(args):
     dom_i = int(np.argmax(stage_sum))
     dom = names[dom_i]
     achieved = {k: alg[k] / (stage_sum[names.index(k)] * 1e-3) / 1e9 for k in names}
-    kernel_key = {"integrate": "k_integrate", "raycast": "k_band_xy+k_band_z+k_ray_fused", "track": "k_icp_iter",
+    kernel_key = {"integrate": "k_integrate", "raycast": "k_band+k_ray_fused", "track": "k_icp_run",
                   "filter": "k_bilateral_batch"}[dom]
     # measured DRAM bytes of one step of the stage: per-unit figures of the
     # committed ncu captures times this workload's units per step
@@ -758,7 +757,9 @@ def run_ours(args):
                 "peak_source": "measured (MEASURED_PEAKS.json hbm_gbs)" if peak_kind == "measured" else
                 "fallback 6800 GB/s",
                 "note": "algorithmic bytes of the stage per step (the first %d timed steps) / its event-timed "
-                        "duration; the ray-cast is issue-bound, not HBM-bound (see profiles/)" % len(stage_steps),
+                        "duration; the ray-cast is issue-bound, not HBM-bound (see profiles/); tracking is counted as "
+                        "28 B for every pixel and scheduled iteration, though it reads the pixels with a valid normal "
+                        "and stops when converged" % len(stage_steps),
                 "algorithmic_bytes_per_step": alg[dom] / len(stage_steps),
                 "stages_gbs": achieved, "stages_frac": {k: v / peak for k, v in achieved.items()}}
     if dom == "raycast":
@@ -1143,7 +1144,7 @@ def run_plain_vga(args):
             "config": vga_config_json(args, world),
             "latency_ms": {"p50": pct(frame_ms, 50), "p99": pct(frame_ms, 99), "max": float(frame_ms.max())},
             "stages_ms": {n_: float(v) for n_, v in zip(names, stage_mean)},
-            "roofline": {"bound": "hbm", "kernel": {"raycast": "k_band_xy+k_band_z+k_ray_fused", "track": "k_icp_iter",
+            "roofline": {"bound": "hbm", "kernel": {"raycast": "k_band+k_ray_fused", "track": "k_icp_run",
                                                     "integrate": "k_integrate", "filter": "k_bilateral_batch"}[dom],
                          "stage": dom, "achieved": achieved[dom], "peak": peak, "unit": "GB/s",
                          "frac": achieved[dom] / peak, "traffic": traffic,

@@ -570,9 +570,9 @@ __device__ void warp_rigid_inverse(const double* T, int lane, double& out) {
 // another's ranges, and an iteration that a session does not need (it
 // converged) costs nothing.  With one launch per iteration every iteration
 // paid the launch, the reads of the tables and the slowest session's closing
-// block: tracking of one 640x480 frame took 307 us in 19 launches and takes
-// 242 us here, with FP64 sums 603 and 440 us; a 640x480 frame 611 -> 545 us, a
-// 320x240 frame 477 -> 427 us.
+// block: tracking of one 640x480 frame took 307 us in 19 launches and 242 when
+// this launch replaced them, with FP64 sums 603 and 440 (146 and 285 now, with
+// the closing and the lists below).
 //
 // Progress needs no block but the running ones: a range is claimed only by a
 // block that then runs it, a closer goes on claiming ranges itself, and a
