@@ -573,8 +573,9 @@ __device__ inline Vol<S> volume_of(const SessionDev& s) {
 // then the shifts within k; and the distances back as bytes.  Bound by the
 // latency of its six steps: 64 x 64 x 64 bricks take 5.5 us (4.8 in blocks of
 // 1024 threads, which halve the slabs in flight: 32 sessions 55 us instead of
-// 38).  Two passes over bytes (the x and y windows of a slab, then the z
-// windows of a row, 15 compares a brick each) took 7.9 + 5.4 and 59 + 24.
+// 38), 40 and 41 bricks a side 4.8 and 6.0.  Two passes over bytes (the x and
+// y windows of a slab, then the z windows of a row, 15 compares a brick each)
+// took 7.9 + 5.4 and 59 + 24 (the two sizes 7.8 and 8.0).
 constexpr int kBandThreads = 512;
 constexpr int kBandSlabs = 2 * kBandReach + 1;
 constexpr int kBandWords = kMaxBricksAxis / 32 * kMaxBricksAxis;  // most words of a slab
@@ -601,31 +602,32 @@ __global__ void __launch_bounds__(kBandThreads) k_band(const BatchTable* __restr
     const float inv_words = 1.0f / (float)words, inv_nw = 1.0f / (float)nw;
     const uint8_t* __restrict__ band = s->band;
     __syncthreads();  // the previous slab's reads are done
-    if (nb0 % 16 == 0) {  // a word's flags are one or two 16-byte reads
-      for (int i = threadIdx.x; i < kBandSlabs * words; i += kBandThreads) {
-        const int dz = small_div(i, inv_words), w = i - dz * words, zz = z + dz - kBandReach;
-        uint32_t bits = 0u;
-        if (zz >= 0 && zz < nb2) {
-          const int y = small_div(w, inv_nw), x = (w - y * nw) * 32;
-          const uint4* src = reinterpret_cast<const uint4*>(band + (size_t)zz * np + y * nb0 + x);
-          const uint4 a = src[0];
+    // a thread per word; its flags in the widest reads that the rows' length
+    // aligns, all in flight together
+    for (int i = threadIdx.x; i < kBandSlabs * words; i += kBandThreads) {
+      const int dz = small_div(i, inv_words), w = i - dz * words, zz = z + dz - kBandReach;
+      uint32_t bits = 0u;
+      if (zz >= 0 && zz < nb2) {
+        const int y = small_div(w, inv_nw), x = (w - y * nw) * 32, left = nb0 - x;
+        const uint8_t* __restrict__ src = band + (size_t)zz * np + y * nb0 + x;
+        if (nb0 % 16 == 0) {
+          const uint4 a = reinterpret_cast<const uint4*>(src)[0];
           bits = pack4(a.x) | pack4(a.y) << 4 | pack4(a.z) << 8 | pack4(a.w) << 12;
-          if (x + 16 < nb0) {
-            const uint4 b = src[1];
+          if (left > 16) {
+            const uint4 b = reinterpret_cast<const uint4*>(src)[1];
             bits |= (pack4(b.x) | pack4(b.y) << 4 | pack4(b.z) << 8 | pack4(b.w) << 12) << 16;
           }
+        } else if (nb0 % 4 == 0) {
+#pragma unroll
+          for (int k = 0; k < 8; k++)
+            if (4 * k < left) bits |= pack4(reinterpret_cast<const uint32_t*>(src)[k]) << (4 * k);
+        } else {
+#pragma unroll
+          for (int k = 0; k < 32; k++)
+            if (k < left) bits |= (uint32_t)src[k] << k;
         }
-        B[dz][w] = bits;
       }
-    } else {  // a warp per word
-      const int lane = threadIdx.x & 31;
-      for (int i = threadIdx.x >> 5; i < kBandSlabs * words; i += kBandThreads / 32) {
-        const int dz = small_div(i, inv_words), w = i - dz * words, zz = z + dz - kBandReach;
-        const int y = small_div(w, inv_nw), x = (w - y * nw) * 32 + lane;
-        const bool in = zz >= 0 && zz < nb2 && x < nb0 && band[(size_t)zz * np + y * nb0 + x];
-        const uint32_t bits = __ballot_sync(0xffffffffu, in);
-        if (lane == 0) B[dz][w] = bits;
-      }
+      B[dz][w] = bits;
     }
     __syncthreads();
     for (int i = threadIdx.x; i < kBandReach * words; i += kBandThreads) {
