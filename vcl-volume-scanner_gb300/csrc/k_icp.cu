@@ -992,13 +992,14 @@ __global__ void __launch_bounds__(kThreads, VS_ICP_MIN_BLOCKS)
     const PT mine = acc.reduce_scatter(lane);
     if (lane < 29) wsum[warp][lane] = mine;
     __syncthreads();
-    // the range again, read back from shared memory: over the pixel loop it
-    // would hold registers
-    const int slot = reload(&s_slot);
-    const unsigned word = reload(&s_word);
-    const SessionDev* sr = reload(&sS[slot]);
-    const int ranges = reload(&sNvb[word >> 30][slot]);
     if (warp == 0) {
+      // the range again, read back from shared memory: over the pixel loop it
+      // would hold registers.  Only this warp reads it here, because its claim
+      // below writes the next one before the other warps pass a barrier.
+      const int slot = reload(&s_slot);
+      const unsigned word = reload(&s_word);
+      const SessionDev* sr = reload(&sS[slot]);
+      const int ranges = reload(&sNvb[word >> 30][slot]);
       if (lane < 29) {
         PT v = wsum[0][lane];
         for (int q = 1; q < kThreads / 32; q++) v = combine(v, wsum[q][lane], MODE);
@@ -1021,7 +1022,12 @@ __global__ void __launch_bounds__(kThreads, VS_ICP_MIN_BLOCKS)
     }
     __syncthreads();
     if (s_close) {
-      // ---- last range of this iteration ----
+      // ---- last range of this iteration: no claim was made, so the range
+      // stands until the one after the closing (and its barrier) ----
+      const int slot = reload(&s_slot);
+      const unsigned word = reload(&s_word);
+      const SessionDev* sr = reload(&sS[slot]);
+      const int ranges = reload(&sNvb[word >> 30][slot]);
       const unsigned next =
           close_iteration<MODE>(sr, ranges, (int)(word >> 30), (int)((word >> 16) & 0x3fffu), frame_mode);
       if (warp == 0) {
