@@ -10,6 +10,8 @@
 #include <string.h>
 
 #include <algorithm>
+#include <functional>
+#include <string>
 #include <thread>
 #include <type_traits>
 #include <vector>
@@ -25,6 +27,9 @@
 #define __launch_bounds__(...)
 #undef __noinline__
 #define __noinline__ __attribute__((noinline))
+
+// called before an atomic operation on a counter (a test may hold a block there)
+extern std::function<void(const void*)> emu_before_atomic;
 
 namespace {
 
@@ -96,6 +101,7 @@ inline T __reduce_add_sync(unsigned, T v) {
 
 template <class T>
 inline T atomicAdd(T* p, T v) {
+  if (emu_before_atomic) emu_before_atomic(p);
   return __atomic_fetch_add(p, v, __ATOMIC_SEQ_CST);
 }
 template <class T>

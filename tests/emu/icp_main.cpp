@@ -1,14 +1,21 @@
-// Runs a block of the tracking kernels on the host: icp_main MODE LISTED
-// prints the outcome of two frames as one JSON line.
+// Runs blocks of the tracking kernels on the host: icp_main SCENARIO MODE
+// LISTED prints the outcome of two frames as one JSON line (alone: one block;
+// idle: a second block that runs out of looks while the first holds a range;
+// stuck: a frame whose iteration nobody ends, then a clean one).
 #include <stdio.h>
 #include <stdlib.h>
+
+#include <condition_variable>
+#include <mutex>
 
 #include "cuda_emu.h"
 #include "vs_internal.cuh"
 
 using namespace vs;
 void emu_begin_a(const BatchTable*, unsigned*, int);
-void emu_track_a(const BatchTable*, unsigned*, int, int, int);
+void emu_track_a(const BatchTable*, unsigned*, int, int);
+void emu_track_b(const BatchTable*, unsigned*, int, int);
+std::function<void(const void*)> emu_before_atomic;
 
 namespace {
 
@@ -87,16 +94,52 @@ struct Scene {
 }  // namespace
 
 int main(int argc, char** argv) {
-  if (argc != 3) return 2;
-  const int mode = atoi(argv[1]);
-  Scene c(atoi(argv[2]) != 0);
+  if (argc != 4) return 2;
+  const std::string what = argv[1];
+  const int mode = atoi(argv[2]);
+  const bool listed = atoi(argv[3]) != 0;
+  Scene c(listed);
+  const int ranges = listed ? (kW * kH + 255) / 256 : kRanges;
   printf("{");
   emu_begin_a(&c.t, c.words(), 1);
-  emu_track_a(&c.t, c.words(), 1, 0, mode);
+  if (what == "alone") {
+    emu_track_a(&c.t, c.words(), 0, mode);
+  } else if (what == "idle") {
+    // the first block is held before the arrival of its first iteration's
+    // last range; the second finds no range, and must leave
+    std::mutex m;
+    std::condition_variable cv;
+    int arrivals = 0;
+    bool held = false, left = false;
+    emu_before_atomic = [&](const void* p) {
+      if (p != &c.counter) return;
+      std::unique_lock<std::mutex> l(m);
+      if (++arrivals != ranges) return;
+      held = true;
+      cv.notify_all();
+      cv.wait(l, [&] { return left; });
+    };
+    std::thread first([&] { emu_track_a(&c.t, c.words(), 0, mode); });
+    {
+      std::unique_lock<std::mutex> l(m);
+      cv.wait(l, [&] { return held; });
+    }
+    emu_track_b(&c.t, c.words(), 1, mode);
+    {
+      std::unique_lock<std::mutex> l(m);
+      left = true;
+      cv.notify_all();
+    }
+    first.join();
+    emu_before_atomic = nullptr;
+  } else {
+    c.t.icp_word[0] += (unsigned)ranges;  // every range taken, by blocks that never arrive
+    emu_track_b(&c.t, c.words(), 1, mode);
+  }
   c.print("frame");
   printf(", ");
   emu_begin_a(&c.t, c.words(), 1);
-  emu_track_a(&c.t, c.words(), 1, 0, mode);
+  emu_track_a(&c.t, c.words(), 0, mode);
   c.print("next");
   printf("}\n");
   return 0;

@@ -1,7 +1,8 @@
 """The block scheduling of the tracking kernels, on the host: k_icp.cu
 compiled with one OS thread per CUDA thread.  Under ThreadSanitizer every
 pair of accesses to a block's shared memory that no barrier orders is an
-error."""
+error; two blocks together show what a block that runs out of looks leaves
+behind."""
 import json
 import os
 import re
@@ -26,32 +27,68 @@ def _host_source(name):
     assert "asm" not in re.sub(r"//.*", "", src)
     if name == "k_icp.cu":
         src = src[:src.index("void launch_gather_heads(")] + "}  // namespace vs\n"
+        src, n = re.subn(r"constexpr int kIdleLimit = [^;]+;", "constexpr int kIdleLimit = 20;", src)
+        assert n == 1
     return src
+
+
+FLAGS = ["g++", "-std=c++17", "-O1", "-g", "-ffp-contract=off", "-w", "-pthread"]
+
+
+def _build(tmp, *extra):
+    for name in ("k_icp.cu", "vs_internal.cuh"):
+        (tmp / name).write_text(_host_source(name))
+    flags = FLAGS + list(extra) + ["-I", str(tmp), "-I", EMU, "-I", os.path.join(ROOT, "include"), "-isystem",
+                                   os.path.join(CUDA, "include"), '-DEMU_ICP="k_icp.cu"']
+    objs = []
+    for tag, src in (("a", "icp_block.cpp"), ("b", "icp_block.cpp"), ("main", "icp_main.cpp")):
+        objs.append(str(tmp / (tag + ".o")))
+        subprocess.run(flags + ["-DEMU_BLOCK=" + tag, "-c", os.path.join(EMU, src), "-o", objs[-1]], check=True)
+    subprocess.run(flags + objs + ["-o", str(tmp / "icp_main")], check=True)
+    return str(tmp / "icp_main")
+
+
+@pytest.fixture(scope="module")
+def plain(tmp_path_factory):
+    return _build(tmp_path_factory.mktemp("icp"))
 
 
 @pytest.fixture(scope="module")
 def checked(tmp_path_factory):
     """the program under ThreadSanitizer"""
     tmp = tmp_path_factory.mktemp("icp_tsan")
-    flags = ["g++", "-std=c++17", "-O1", "-g", "-ffp-contract=off", "-w", "-pthread", "-fsanitize=thread"]
     (tmp / "probe.cpp").write_text("int main() { return 0; }\n")
     probe = str(tmp / "probe")
-    if subprocess.run(flags + [str(tmp / "probe.cpp"), "-o", probe]).returncode or subprocess.run([probe]).returncode:
+    cmd = FLAGS + ["-fsanitize=thread", str(tmp / "probe.cpp"), "-o", probe]
+    if subprocess.run(cmd).returncode or subprocess.run([probe]).returncode:
         pytest.skip("ThreadSanitizer does not run here")
-    for name in ("k_icp.cu", "vs_internal.cuh"):
-        (tmp / name).write_text(_host_source(name))
-    flags += ["-I", str(tmp), "-I", EMU, "-I", os.path.join(ROOT, "include"), "-isystem",
-              os.path.join(CUDA, "include"), "-DEMU_BLOCK=a", '-DEMU_ICP="k_icp.cu"']
-    exe = str(tmp / "icp_main")
-    subprocess.run(flags + [os.path.join(EMU, f) for f in ("icp_block.cpp", "icp_main.cpp")] + ["-o", exe],
-                   check=True)
-    return exe
+    return _build(tmp, "-fsanitize=thread")
+
+
+def _run(exe, scenario, mode, listed):
+    r = subprocess.run([exe, scenario, str(mode), str(int(listed))], capture_output=True, text=True, timeout=300)
+    assert "data race" not in r.stderr, r.stderr[:3000]
+    assert r.returncode == 0, r.stderr[:3000]
+    return json.loads(r.stdout)
 
 
 @pytest.mark.parametrize("mode,listed", [(KAHAN, False), (KAHAN, True), (FP64, True)])
 def test_shared_memory_is_ordered(checked, mode, listed):
-    r = subprocess.run([checked, str(mode), str(int(listed))], capture_output=True, text=True, timeout=300)
-    assert "data race" not in r.stderr, r.stderr[:3000]
-    assert r.returncode == 0, r.stderr[:3000]
-    out = json.loads(r.stdout)
+    out = _run(checked, "alone", mode, listed)
     assert [out[f]["tracked"] for f in ("frame", "next")] == [1, 1]
+
+
+@pytest.mark.parametrize("listed", [False, True])
+def test_block_that_runs_out_of_looks_changes_nothing(plain, listed):
+    """a block leaves while another holds the iteration's last range: the frame
+    ends as it does with that block alone"""
+    assert _run(plain, "idle", KAHAN, listed) == _run(plain, "alone", KAHAN, listed)
+
+
+def test_iteration_that_nobody_ends(plain):
+    """its frame is lost, counted and leaves the pose; the next one is tracked
+    as if it were the first"""
+    alone, out = _run(plain, "alone", KAHAN, False), _run(plain, "stuck", KAHAN, False)
+    eye = [float(k % 5 == 0) for k in range(16)]
+    assert out["frame"] == dict(tracked=0, failed=1, frame=2, iters=0, count=0, T_gc=eye)
+    assert out["next"] == dict(alone["frame"], frame=3)

@@ -580,9 +580,11 @@ __device__ void warp_rigid_inverse(const double* T, int lane, double& out) {
 // time.  It leaves when every session is done, or when the unfinished
 // sessions could not give it a range (blocks are numbered, and the block's
 // number is not below the sum of their largest range counts), which frees its
-// SM for other streams' kernels.
+// SM for other streams' kernels, or when it has looked kIdleLimit times.  A
+// session's outcome is written by the block that ends its tracking alone: until
+// then its frame counts as lost, and stays so if nobody ends it.
 constexpr unsigned kWordDone = 3u;
-constexpr int kIdleLimit = 1 << 22;  // looks without a range before a block gives up (seconds; none in a sound run)
+constexpr int kIdleLimit = 1 << 22;  // looks without a range before a block leaves (seconds; none in a sound run)
 
 __device__ __forceinline__ unsigned work_word(int level, int iter) {
   return ((unsigned)level << 30) | ((unsigned)iter << 16);
@@ -596,8 +598,8 @@ __device__ inline int next_level(const SessionDev* s, int l) {
 }
 
 // end of a session's tracking, one warp: T_gc <- T12 T_gc unless it failed
-// or was skipped
-__device__ void icp_finish(Pose* P, bool skip, bool failed, int frame_mode, int ln, double* Tn, double* A) {
+// or was skipped, and the outcome
+__device__ void icp_finish(Pose* P, bool skip, bool failed, int ln, double* Tn, double* A) {
   if (!skip && !failed) {
     if (ln < 16) A[ln] = __ldcg(&P->T12[ln]);
     __syncwarp();
@@ -613,13 +615,13 @@ __device__ void icp_finish(Pose* P, bool skip, bool failed, int frame_mode, int 
   }
   if (ln == 0) {
     P->tracked = failed ? 0 : 1;
-    if (frame_mode) P->frame += 1;
+    P->failed = failed ? 1 : 0;
   }
 }
 
 // one warp per slot: the increment of this frame starts at identity (or at
-// `init`, and then only level 0 runs), and the session's first iteration is
-// published
+// `init`, and then only level 0 runs), its frame is counted, as lost until its
+// tracking ends, and the session's first iteration is published
 __global__ void k_icp_begin(const BatchTable* __restrict__ bt, unsigned* words, int frame_mode, int with_init,
                             const float* init) {
   if ((int)blockIdx.x >= bt->n) return;
@@ -638,12 +640,16 @@ __global__ void k_icp_begin(const BatchTable* __restrict__ bt, unsigned* words, 
   }
   const int l = skip ? -1 : next_level(s, with_init ? 0 : s->levels - 1);
   __syncwarp();
-  if (l < 0) icp_finish(P, skip, false, frame_mode, ln, Tn, A);
   if (ln == 0) {
     P->skip = skip ? 1 : 0;
-    P->failed = 0;
+    P->tracked = 0;
+    P->failed = 1;
+    if (frame_mode) P->frame += 1;
     P->iters_run = 0;
     P->valid_count = 0;
+  }
+  if (l < 0) icp_finish(P, skip, false, ln, Tn, A);
+  if (ln == 0) {
     *s->icp_counter = 0u;
     words[blockIdx.x] = l < 0 ? kWordDone << 30 : work_word(l, 0);
   }
@@ -653,8 +659,7 @@ __global__ void k_icp_begin(const BatchTable* __restrict__ bt, unsigned* words, 
 // closing block together.  Warp 1 decides failure and records the
 // sums; warp 0 solves, updates the pose and returns the session's next work
 // word (to be published once its lanes' writes are out).
-__device__ __forceinline__ unsigned icp_close(const SessionDev* s, const double* fin, int level, int iter,
-                                           int frame_mode) {
+__device__ __forceinline__ unsigned icp_close(const SessionDev* s, const double* fin, int level, int iter) {
   __shared__ double A[16], Tn[16];
   __shared__ float xf[6];
   __shared__ int status;
@@ -727,10 +732,8 @@ __device__ __forceinline__ unsigned icp_close(const SessionDev* s, const double*
     const int l = next_level(s, level - 1);
     if (l >= 0) return work_word(l, 0);
     __syncwarp();
-  } else if (ln == 0) {
-    P->failed = 1;
   }
-  icp_finish(P, false, failed, frame_mode, ln, Tn, A);
+  icp_finish(P, false, failed, ln, Tn, A);
   return kWordDone << 30;
 }
 
@@ -740,7 +743,7 @@ __device__ __forceinline__ unsigned icp_close(const SessionDev* s, const double*
 // then the solve.  Warp 0 receives the next work word, with every write of
 // the block visible to whoever reads that word after a fence.
 template <int MODE>
-__device__ __noinline__ unsigned close_iteration(const SessionDev* s, int nvb, int level, int iter, int frame_mode) {
+__device__ __noinline__ unsigned close_iteration(const SessionDev* s, int nvb, int level, int iter) {
   typedef typename PartT<MODE>::type PT;
   __shared__ double fin[29];
   // 8 threads per quantity, each a fixed stride over the ranges, then a fixed
@@ -771,7 +774,7 @@ __device__ __noinline__ unsigned close_iteration(const SessionDev* s, int nvb, i
   if (k < 29 && j == 0) fin[k] = (double)v.x + (double)v.y;
   __syncthreads();
   unsigned next = 0u;
-  if (threadIdx.x < 64) next = icp_close(s, fin, level, iter, frame_mode);
+  if (threadIdx.x < 64) next = icp_close(s, fin, level, iter);
   if (threadIdx.x < 32) {
     __syncwarp();
     __threadfence();
@@ -788,9 +791,8 @@ __device__ __noinline__ unsigned close_iteration(const SessionDev* s, int nvb, i
 // on (prefer) while that has ranges; otherwise it takes the first session that
 // does, so that few sessions are under way at a time and their maps stay in
 // L2 over their iterations.
-__device__ __noinline__ void claim_range(unsigned* __restrict__ words, int n, const SessionDev* const* sS,
-                                         const int (*sNvb)[kMaxSlots], int prefer, int* out_slot,
-                                         unsigned* out_word) {
+__device__ __noinline__ void claim_range(unsigned* __restrict__ words, int n, const int (*sNvb)[kMaxSlots],
+                                         int prefer, int* out_slot, unsigned* out_word) {
   const int lane = threadIdx.x & 31;
   int slot = -1;
   unsigned w = 0u;
@@ -809,13 +811,7 @@ __device__ __noinline__ void claim_range(unsigned* __restrict__ words, int n, co
       }
       need = __reduce_add_sync(0xffffffffu, need);
       if (first < 0) {
-        if ((int)blockIdx.x >= need) break;
-        if (look >= kIdleLimit) {
-          // an iteration that does not end: its frame counts as lost
-          for (int q = lane; q < n; q += 32)
-            if ((load_word(words + q) >> 30) != kWordDone) sS[q]->pose->failed = 1, sS[q]->pose->tracked = 0;
-          break;
-        }
+        if ((int)blockIdx.x >= need || look >= kIdleLimit) break;
         __nanosleep(40);
         continue;
       }
@@ -865,7 +861,7 @@ __device__ __forceinline__ T reload(const T* p) {
 
 template <int MODE>
 __global__ void __launch_bounds__(kThreads, VS_ICP_MIN_BLOCKS)
-    k_icp_run(const BatchTable* __restrict__ bt, unsigned* __restrict__ words, int frame_mode) {
+    k_icp_run(const BatchTable* __restrict__ bt, unsigned* __restrict__ words) {
   typedef typename PartT<MODE>::type PT;
   __shared__ PT wsum[kThreads / 32][29];
   __shared__ float sT21[12], sK[4];
@@ -889,7 +885,7 @@ __global__ void __launch_bounds__(kThreads, VS_ICP_MIN_BLOCKS)
   }
   __syncthreads();
 
-  auto claim = [&](int prefer) { claim_range(words, n, sS, sNvb, prefer, &s_slot, &s_word); };
+  auto claim = [&](int prefer) { claim_range(words, n, sNvb, prefer, &s_slot, &s_word); };
   if (warp == 0) claim(-1);
   __syncthreads();
   while (s_slot >= 0) {
@@ -1028,8 +1024,7 @@ __global__ void __launch_bounds__(kThreads, VS_ICP_MIN_BLOCKS)
       const unsigned word = reload(&s_word);
       const SessionDev* sr = reload(&sS[slot]);
       const int ranges = reload(&sNvb[word >> 30][slot]);
-      const unsigned next =
-          close_iteration<MODE>(sr, ranges, (int)(word >> 30), (int)((word >> 16) & 0x3fffu), frame_mode);
+      const unsigned next = close_iteration<MODE>(sr, ranges, (int)(word >> 30), (int)((word >> 16) & 0x3fffu));
       if (warp == 0) {
         if (lane == 0) atomicExch(words + slot, next);
         claim((next >> 30) == kWordDone ? -1 : slot);
@@ -1112,8 +1107,7 @@ void launch_icp(const BatchTable* bt, int reduce_mode, cudaStream_t st, bool fra
   // (zz_flag_track, z_yooji_object_scanner.cpp:534,572-576); explicit
   // tp_Track_Pose calls always track
   unsigned* words = const_cast<unsigned*>(bt->icp_word);
-  const int fm = frame_mode ? 1 : 0;
-  k_icp_begin<<<kMaxSlots, 32, 0, st>>>(bt, words, fm, init_T12 ? 1 : 0, init_T12);
+  k_icp_begin<<<kMaxSlots, 32, 0, st>>>(bt, words, frame_mode ? 1 : 0, init_T12 ? 1 : 0, init_T12);
   // Two of the three blocks that fit an SM: the rest of each SM takes the
   // other branch's kernels while this launch waits for a closer.  (Sixteen
   // sessions, two branches: 1955 us per step with three blocks, 1894 with
@@ -1122,13 +1116,13 @@ void launch_icp(const BatchTable* bt, int reduce_mode, cudaStream_t st, bool fra
   const int grid = sm_count() * 2;
   switch (reduce_mode) {
     case VS_REDUCE_FP32:
-      k_icp_run<VS_REDUCE_FP32><<<grid, kThreads, 0, st>>>(bt, words, fm);
+      k_icp_run<VS_REDUCE_FP32><<<grid, kThreads, 0, st>>>(bt, words);
       break;
     case VS_REDUCE_FP64:
-      k_icp_run<VS_REDUCE_FP64><<<grid, kThreads, 0, st>>>(bt, words, fm);
+      k_icp_run<VS_REDUCE_FP64><<<grid, kThreads, 0, st>>>(bt, words);
       break;
     default:
-      k_icp_run<VS_REDUCE_KAHAN><<<grid, kThreads, 0, st>>>(bt, words, fm);
+      k_icp_run<VS_REDUCE_KAHAN><<<grid, kThreads, 0, st>>>(bt, words);
       break;
   }
 }

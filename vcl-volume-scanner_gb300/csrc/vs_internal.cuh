@@ -41,7 +41,7 @@ struct Pose {
   float T21[16];       // float inverse of T12, read by the ICP term kernel
   double T_gc[16];     // FP64 master pose, global -> camera
   double T12[16];      // ICP increment of the current frame (camera t0 -> t1)
-  int failed;          // 6x6 system singular this frame
+  int failed;          // no pose this frame: 6x6 system singular, or its tracking did not end
   int skip;            // no tracking this frame (first frame)
   float last_x[6];
   double last_sums[29];
