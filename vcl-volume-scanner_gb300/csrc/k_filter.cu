@@ -624,8 +624,8 @@ void launch_bilateral_float(const SessionDev& h, const float* in, float* out, cu
         <<<dim3(cols, (rows + kPerThread - 1) / kPerThread), dim3(BX, BY), 0, st>>>(in, out, W, H);
 }
 
-void configure_filter_kernels() {
-  cudaFuncSetAttribute(k_inmap_scan, cudaFuncAttributeMaxDynamicSharedMemorySize, kScanSmem);
+cudaError_t configure_filter_kernels() {
+  return cudaFuncSetAttribute(k_inmap_scan, cudaFuncAttributeMaxDynamicSharedMemorySize, kScanSmem);
 }
 
 // work-item prefixes of a batch; host_recs are the host copies of the

@@ -1095,11 +1095,13 @@ int icp_blocks(int npix, int level) {
 // 1302 -> 1172 and 1766 -> 1655 us; of 1 and 64 the same.  (15 and 25 % the same
 // within 1 %; 60 and 100 % leave L1 too little, 1.5 and 3 % more with one
 // session or 64 of them.)
-void configure_icp_kernels() {
+cudaError_t configure_icp_kernels() {
   constexpr int kShared = 40;
-  cudaFuncSetAttribute(k_icp_run<VS_REDUCE_FP32>, cudaFuncAttributePreferredSharedMemoryCarveout, kShared);
-  cudaFuncSetAttribute(k_icp_run<VS_REDUCE_KAHAN>, cudaFuncAttributePreferredSharedMemoryCarveout, kShared);
-  cudaFuncSetAttribute(k_icp_run<VS_REDUCE_FP64>, cudaFuncAttributePreferredSharedMemoryCarveout, kShared);
+  for (auto k : {k_icp_run<VS_REDUCE_FP32>, k_icp_run<VS_REDUCE_KAHAN>, k_icp_run<VS_REDUCE_FP64>}) {
+    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, kShared);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
 }
 
 void launch_icp(const BatchTable* bt, int reduce_mode, cudaStream_t st, bool frame_mode, const float* init_T12) {

@@ -14,19 +14,19 @@
 #include <cstddef>
 #include <cstdio>
 #include <cstring>
-#include <mutex>
 #include <string>
 #include <vector>
 
 #include "vs.h"
+#include "vs_device_once.h"
 #include "vs_host.h"
 #include "vs_internal.cuh"
 
 namespace vs {
 void launch_volume_slab(const SessionDev& h, bool do_export, int z0, int nz, float* tsdf, uint16_t* w,
                         cudaStream_t st);
-void configure_filter_kernels();
-void configure_icp_kernels();
+cudaError_t configure_filter_kernels();
+cudaError_t configure_icp_kernels();
 int integrate_max_dim();
 int integrate_max_image();
 }  // namespace vs
@@ -221,7 +221,7 @@ int build_graph(vs_session* s) {
   return VS_OK;
 }
 
-std::once_flag g_once;
+OncePerDevice g_kernels_configured;
 
 }  // namespace
 
@@ -299,13 +299,15 @@ int vs_session_create(const vs_config* cfg, vs_session** out) {
   int ndev = 0;
   cudaError_t e = cudaGetDeviceCount(&ndev);
   if (e != cudaSuccess || ndev == 0) return fail(VS_ERR_CUDA, "no CUDA device available");
-  std::call_once(g_once, [] {
-    configure_filter_kernels();
-    configure_icp_kernels();
-  });
+  int device = 0;
+  VS_CU(cudaGetDevice(&device));
+  VS_CU(g_kernels_configured.run(device, [] {
+    const cudaError_t f = configure_filter_kernels();
+    return f == cudaSuccess ? configure_icp_kernels() : f;
+  }));
   vs_session* s = new vs_session;
   s->cfg = *cfg;
-  cudaGetDevice(&s->device);
+  s->device = device;
   std::memset(&s->h, 0, sizeof(s->h));
   fill_geometry(cfg, s->h);
   SessionDev& h = s->h;

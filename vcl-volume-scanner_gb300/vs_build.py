@@ -23,7 +23,7 @@ CU_SOURCES = [
     "k_filter.cu", "k_icp.cu", "k_integrate.cu", "k_raycast.cu", "k_mesh.cu", "vs_api.cu", "vs_batch.cu",
     "vs_server.cu", "vs_snapshot.cu", "vs_noalloc.cu", "k_register.cu",
 ]
-HEADERS = ["vs_internal.cuh", "vs_host.h"]
+HEADERS = ["vs_internal.cuh", "vs_host.h", "vs_device_once.h"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_103a,code=sm_103a",
     "-O3", "-lineinfo", "-std=c++17", "-fmad=false",
