@@ -52,7 +52,7 @@ __device__ __forceinline__ float exp2_approx(float x) {
 // the reference's order with its roundings.  A tap that is not above 0 is stored as
 // -infinity: as the centre it makes the sum infinite, elsewhere its weight is
 // 0 and their product not a number.
-template <int R, int P>
+template <bool FROM_MM, int R, int P>
 __device__ inline void bilateral_px(const BilateralSmem<R, P>& m, int tx, int ty0, bool finite, float out[P]) {
   // The Gaussian of delta 4 (:275-286), exp(-x^2 / (2 * 4^2)).  The range
   // weight's exponent is -mod / (2 sigma_r^2), 2 sigma_r^2 = 2.0f * 0.1f *
@@ -100,7 +100,10 @@ __device__ inline void bilateral_px(const BilateralSmem<R, P>& m, int tx, int ty
     out[r] = t[r] / sum[r];
     if (!(t[r] >= 0.0f)) {
       bool hole = finite;  // finite inputs: only a hole gives this
+      // (a frame of units comes here with an unusual scale only: unrolled, the
+      // search would take 72 registers instead of 40 for every frame)
       if (!finite)
+#pragma unroll FROM_MM ? 1 : 25
         for (int i = 0; i < 25; i++) hole |= m.tap[ty0 + r + i / 5][tx + i % 5] == __int_as_float(0xff800000);
       if (hole) out[r] = 0.0f;
     }
@@ -150,7 +153,9 @@ __device__ inline void bilateral_tile(BilateralSmem<R, P>& m, const uint16_t* __
   const int x = x0 + tx, yb = y0 + ty * P;
   if (x < W && yb < H) {
     float f[P];
-    bilateral_px(m, tx, ty * P, FROM_MM, f);
+    // scaled units are finite, and so are the sums of their taps, unless the
+    // session's scale itself is out of range (65535 units of 1e30 are 6.6e34)
+    bilateral_px<FROM_MM>(m, tx, ty * P, FROM_MM && fabsf(scale) <= 1.0e30f, f);
 #pragma unroll
     for (int r = 0; r < P; r++) {
       if (yb + r >= H) break;
