@@ -541,14 +541,33 @@ def ate_all_sessions(specs, ours, ours_tracked, warm_depth, steps):
 # our arm
 # ---------------------------------------------------------------------------
 def stage_bytes(cfg, st):
-    """algorithmic bytes per frame and stage (st: active sub-cubes, voxels updated)"""
+    """algorithmic bytes per frame and stage (st: active sub-cubes, voxels
+    updated).  Tracking has none here: it is a chain of iterations bound by
+    latency, which reads the pixels with a valid normal and stops when
+    converged, so bytes of every pixel and scheduled iteration would count
+    work that it leaves out as bandwidth."""
     W, H = cfg.width, cfg.height
     lv = [(W >> l) * (H >> l) for l in range(3)]
-    it = MIX["icp_iters"]
     return {"filter": 6.0 * W * H + sum(lv[l] * (4 + 4 + 32) for l in range(3)),
-            "track": sum(28.0 * lv[l] * it[l] for l in range(3)),
             "integrate": 4.0 * 512 * st[0] + 4.0 * st[1] + 2.0 * W * H + 8.0 * st[0],
             "raycast": 28.0 * sum(lv)}
+
+
+KERNELS = {"filter": "k_bilateral_batch", "track": "k_icp_run", "integrate": "k_integrate",
+           "raycast": "k_band+k_ray_fused"}
+
+
+def stage_roofline(stage, bytes_, ms, peak, peak_kind, traffic):
+    """the roofline entry of a stage: its counted bytes over its time against
+    the copy bandwidth, or, for a stage without counted bytes, that latency
+    bounds it (bytes_, ms: per stage, of the same frames)"""
+    achieved = {k: b / (ms[k] * 1e-3) / 1e9 for k, b in bytes_.items()}
+    got = achieved.get(stage)
+    return {"bound": "latency" if got is None else "hbm", "kernel": KERNELS[stage], "stage": stage, "achieved": got,
+            "peak": peak, "unit": "GB/s", "frac": None if got is None else got / peak, "traffic": traffic,
+            "peak_source": "measured (MEASURED_PEAKS.json hbm_gbs)" if peak_kind == "measured" else
+            "fallback 6800 GB/s",
+            "stages_gbs": achieved, "stages_frac": {k: v / peak for k, v in achieved.items()}}
 
 
 def run_ours(args):
@@ -647,7 +666,7 @@ def run_ours(args):
     batch.set_stage_timing(True)
     stage_steps = window[:20]
     stage = np.zeros((len(stage_steps), 4))
-    alg = {k: 0.0 for k in ("filter", "track", "integrate", "raycast")}
+    alg = {k: 0.0 for k in ("filter", "integrate", "raycast")}
     for j, r in enumerate(stage_steps):
         batch.step(handles[r], ptrs[r], st.cuda_stream)
         batch.sync()
@@ -732,9 +751,6 @@ def run_ours(args):
     peak, peak_kind = measured_peak_hbm()
     dom_i = int(np.argmax(stage_sum))
     dom = names[dom_i]
-    achieved = {k: alg[k] / (stage_sum[names.index(k)] * 1e-3) / 1e9 for k in names}
-    kernel_key = {"integrate": "k_integrate", "raycast": "k_band+k_ray_fused", "track": "k_icp_run",
-                  "filter": "k_bilateral_batch"}[dom]
     # measured DRAM bytes of one step of the stage: per-unit figures of the
     # committed ncu captures times this workload's units per step
     rays = np.mean([sum(sum(level_pixels(seqs[i]["cfg"])) for i in members[r]) for r in stage_steps])
@@ -749,19 +765,15 @@ def run_ours(args):
         if px is not None:
             traffic = px * np.mean([sum(sum(p * it for p, it in zip(level_pixels(seqs[i]["cfg"]), MIX["icp_iters"]))
                                         for i in members[r]) for r in stage_steps])
-    roofline = {"bound": "hbm", "kernel": kernel_key, "stage": dom,
-                "achieved": achieved[dom], "peak": peak, "unit": "GB/s", "frac": achieved[dom] / peak,
-                "traffic": traffic,
-                "traffic_note": "DRAM bytes per step: bytes per unit from profiles/ncu_traffic.txt x units per step "
-                                "(%.0f rays, %.0f sub-cubes)" % (rays, bricks),
-                "peak_source": "measured (MEASURED_PEAKS.json hbm_gbs)" if peak_kind == "measured" else
-                "fallback 6800 GB/s",
-                "note": "algorithmic bytes of the stage per step (the first %d timed steps) / its event-timed "
-                        "duration; the ray-cast is issue-bound, not HBM-bound (see profiles/); tracking is counted as "
-                        "28 B for every pixel and scheduled iteration, though it reads the pixels with a valid normal "
-                        "and stops when converged" % len(stage_steps),
-                "algorithmic_bytes_per_step": alg[dom] / len(stage_steps),
-                "stages_gbs": achieved, "stages_frac": {k: v / peak for k, v in achieved.items()}}
+    roofline = stage_roofline(dom, alg, dict(zip(names, stage_sum)), peak, peak_kind, traffic)
+    achieved = roofline["stages_gbs"]
+    roofline.update({
+        "traffic_note": "DRAM bytes per step: bytes per unit from profiles/ncu_traffic.txt x units per step "
+                        "(%.0f rays, %.0f sub-cubes)" % (rays, bricks),
+        "note": "algorithmic bytes of the stage per step (the first %d timed steps) / its event-timed duration; the "
+                "ray-cast is issue-bound, not HBM-bound (see profiles/); tracking is bound by latency and has no "
+                "counted bytes" % len(stage_steps),
+        "algorithmic_bytes_per_step": alg[dom] / len(stage_steps) if dom in alg else None})
     if dom == "raycast":
         # the ray-cast's own bound is instruction issue: warp instructions per
         # ray from the committed ncu captures times this workload's rays, over
@@ -1098,7 +1110,6 @@ def run_plain_vga(args):
     st_ = (stats[:, 0].mean(), stats[:, 1].mean())
     alg = stage_bytes(cfg, st_)
     dom = names[int(np.argmax(stage_mean))]
-    achieved = {k: alg[k] / (stage_mean[names.index(k)] * 1e-3) / 1e9 for k in names}
     rays = sum(level_pixels(cfg))
     traffic = None
     if dom == "raycast":
@@ -1109,6 +1120,8 @@ def run_plain_vga(args):
         px = traffic_per_unit("k_icp_iter", "dram_bytes_per_pixel")
         if px is not None:
             traffic = px * sum(p * it for p, it in zip(level_pixels(cfg), VGA["icp_iters"]))
+    roofline = stage_roofline(dom, alg, dict(zip(names, stage_mean)), peak, peak_kind, traffic)
+    achieved = roofline["stages_gbs"]
     cpu = ate = None
     if not args.no_cpu:
         import oracle_py as O
@@ -1144,12 +1157,7 @@ def run_plain_vga(args):
             "config": vga_config_json(args, world),
             "latency_ms": {"p50": pct(frame_ms, 50), "p99": pct(frame_ms, 99), "max": float(frame_ms.max())},
             "stages_ms": {n_: float(v) for n_, v in zip(names, stage_mean)},
-            "roofline": {"bound": "hbm", "kernel": {"raycast": "k_band+k_ray_fused", "track": "k_icp_run",
-                                                    "integrate": "k_integrate", "filter": "k_bilateral_batch"}[dom],
-                         "stage": dom, "achieved": achieved[dom], "peak": peak, "unit": "GB/s",
-                         "frac": achieved[dom] / peak, "traffic": traffic,
-                         "peak_source": "measured (MEASURED_PEAKS.json hbm_gbs)" if peak_kind == "measured" else
-                         "fallback 6800 GB/s", "stages_gbs": achieved},
+            "roofline": roofline,
             "integrate": {"active_subcubes": st_[0], "voxels_updated": st_[1],
                           "achieved_gbs": achieved["integrate"], "frac": achieved["integrate"] / peak},
             "cpu_baseline": cpu,
