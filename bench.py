@@ -970,7 +970,7 @@ def serving_sweeps(V, seqs, host, sessions, span_s):
 # ---------------------------------------------------------------------------
 VGA = dict(name="plain_vga_512", width=640, height=480, fx=525.0, fy=525.0, cx=319.5, cy=239.5, volume=512,
            size_m=1.5, mu=0.02, icp_iters=(10, 5, 4), th_icp=0.1 ** 2, normal_deg=20.0, dropout_blob=0.015,
-           max_depth=2.5, seed=2)
+           max_depth=2.5, seed=2, ate_frames=12)
 L2_FLUSH_BYTES = 256 << 20
 
 
@@ -1137,7 +1137,7 @@ def run_plain_vga(args):
         cpu = {"value": n / dt, "unit": "frames/s", "cores": 1, "kind": "port",
                "sample": "first %d frames of the sequence (%.1f s), oracle port, reference FP32 semantics, 1 thread"
                          % (n, dt)}
-        nf = min(n, args.ate_frames)
+        nf = min(n, VGA["ate_frames"])
         set_omp_threads(os.cpu_count() or 1)
         s64 = O.Session(O.config_from_vs(cfg, reduce_mode=3, tsdf_store=0), f64=True)
         s2 = V.Session(cfg)
