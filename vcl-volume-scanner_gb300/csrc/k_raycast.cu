@@ -812,11 +812,11 @@ __device__ inline void shade_ray(const RayArgs& a, const Vol<S>& V, const Sessio
 }
 
 // phase 2: the maps of every ray from its surface point in the hit buffer
-template <class S, bool COLOR>
+template <class S>
 __global__ void __launch_bounds__(kRayThreads, VS_SHADE_MIN_BLOCKS) k_ray_shade(RayArgs a) {
   for_each_ray_tile<false>(a, [&](const SessionDev& s, int l, int x, int y, const TileCam& c) {
     const float4 h = s.ray_hit[hit_offset(s, l) + (size_t)y * s.lv[l].W + x];
-    shade_ray<S, COLOR>(a, volume_of<S>(s), s, c, l, x, y, h.w != 0.0f, f3(h.x, h.y, h.z));
+    shade_ray<S, true>(a, volume_of<S>(s), s, c, l, x, y, h.w != 0.0f, f3(h.x, h.y, h.z));
   });
 }
 
@@ -869,11 +869,14 @@ int max_per_sm(K kernel) {
   return per_sm;
 }
 
+// of the march grid (with the shading in it, unless a session keeps colour)
+// and the shading grid
 template <class S>
-int ray_max_per_sm(bool shade) {
+int ray_max_per_sm(bool shade, bool color) {
+  static const int f = max_per_sm(k_ray_fused<S, false>);
   static const int m = max_per_sm(k_ray_march<S, false>);
-  static const int h = max_per_sm(k_ray_shade<S, false>);
-  return shade ? h : m;
+  static const int h = max_per_sm(k_ray_shade<S>);
+  return shade ? h : color ? m : f;
 }
 
 int grid_of(int want, int most) { return sm_count() * ((want > 0 && want < most) ? want : most); }
@@ -882,24 +885,20 @@ template <class S>
 void launch_ray_phases(const RayArgs& a0, const LaunchShape& shape, bool color, cudaStream_t st) {
   RayArgs a = a0;
   k_band<<<sm_count() * 4, kBandThreads, 0, st>>>(a.bt);
+  const int march = grid_of(shape.march_blocks_per_sm, ray_max_per_sm<S>(false, color));
   if (!color) {
-    static const int most_fused = max_per_sm(k_ray_fused<S, false>);
     if (a.mode & kRayScene)
-      k_ray_fused<S, true><<<grid_of(shape.march_blocks_per_sm, most_fused), kRayThreads, 0, st>>>(a);
+      k_ray_fused<S, true><<<march, kRayThreads, 0, st>>>(a);
     else
-      k_ray_fused<S, false><<<grid_of(shape.march_blocks_per_sm, most_fused), kRayThreads, 0, st>>>(a);
+      k_ray_fused<S, false><<<march, kRayThreads, 0, st>>>(a);
     return;
   }
   if (a.mode & kRayScene)
-    k_ray_march<S, true><<<grid_of(shape.march_blocks_per_sm, ray_max_per_sm<S>(false)), kRayThreads, 0, st>>>(a);
+    k_ray_march<S, true><<<march, kRayThreads, 0, st>>>(a);
   else
-    k_ray_march<S, false><<<grid_of(shape.march_blocks_per_sm, ray_max_per_sm<S>(false)), kRayThreads, 0, st>>>(a);
-  a.work = a0.work + 4;
-  static const int most_color = max_per_sm(k_ray_shade<S, true>);
-  if (color)
-    k_ray_shade<S, true><<<grid_of(shape.shade_blocks_per_sm, most_color), kRayThreads, 0, st>>>(a);
-  else
-    k_ray_shade<S, false><<<grid_of(shape.shade_blocks_per_sm, ray_max_per_sm<S>(true)), kRayThreads, 0, st>>>(a);
+    k_ray_march<S, false><<<march, kRayThreads, 0, st>>>(a);
+  a.work = a0.work + 2;
+  k_ray_shade<S><<<grid_of(shape.shade_blocks_per_sm, ray_max_per_sm<S>(true, color)), kRayThreads, 0, st>>>(a);
 }
 
 void launch_raycast(const BatchTable* bt, int tsdf_type, int level, const float* Tgc, const float* Tcg,
@@ -908,7 +907,7 @@ void launch_raycast(const BatchTable* bt, int tsdf_type, int level, const float*
                     bool color, int mode) {
   RayArgs a;
   a.bt = bt;
-  a.work = const_cast<unsigned*>(bt->work);  // [0..1] march, [4..5] shade
+  a.work = const_cast<unsigned*>(bt->work);  // [0..1] march, [2..3] shade
   a.level = level;
   a.Tgc = Tgc;
   a.Tcg = Tcg;
@@ -936,14 +935,14 @@ void launch_raycast(const BatchTable* bt, int tsdf_type, int level, const float*
   }
 }
 
-int ray_max_blocks_per_sm(int tsdf_type, bool shade) {
+int ray_max_blocks_per_sm(int tsdf_type, bool shade, bool color) {
   switch (tsdf_type) {
     case VS_TSDF_FP16:
-      return ray_max_per_sm<StoreF16>(shade);
+      return ray_max_per_sm<StoreF16>(shade, color);
     case VS_TSDF_FP32:
-      return ray_max_per_sm<StoreF32>(shade);
+      return ray_max_per_sm<StoreF32>(shade, color);
     default:
-      return ray_max_per_sm<StoreI16>(shade);
+      return ray_max_per_sm<StoreI16>(shade, color);
   }
 }
 

@@ -524,7 +524,8 @@ int vs_batch_autotune(vs_batch* b, vs_session* const* sessions, int n, int reps,
     hr[i] = &sessions[i]->h;
     dr[i] = sessions[i]->d;
   }
-  const int most_m = ray_max_blocks_per_sm(k.tsdf_type, false), most_s = ray_max_blocks_per_sm(k.tsdf_type, true);
+  const int most_m = ray_max_blocks_per_sm(k.tsdf_type, false, k.color != 0),
+            most_s = ray_max_blocks_per_sm(k.tsdf_type, true, k.color != 0);
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   cudaError_t e = cudaEventCreate(&e0);
   if (e == cudaSuccess) e = cudaEventCreate(&e1);

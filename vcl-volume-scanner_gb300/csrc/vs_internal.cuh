@@ -131,7 +131,7 @@ struct BatchTable {
                                        // memory, or pinned host memory the device can address; the ingest
                                        // also copies it into the session's frame buffer); NULL: that buffer
   int slab[kMaxSlots + 1];             // z slabs of bricks (band distance)
-  unsigned work[8];                    // work counters ([0..1] ray march, [4..5] ray shading); zero between
+  unsigned work[4];                    // work counters ([0..1] ray march, [2..3] ray shading); zero between
                                        // launches
   unsigned icp_word[kMaxSlots];        // per slot: level, iteration and next range of its tracking (k_icp.cu)
 };
@@ -319,7 +319,7 @@ int icp_blocks(int npix, int level);
 int sm_count();
 void fill_batch_table(BatchTable& hb, const SessionDev* const* host_recs, const SessionDev* const* dev_recs, int n,
                       int ray_lx = 3, int bil_rows = 8);
-int ray_max_blocks_per_sm(int tsdf_type, bool shade);
+int ray_max_blocks_per_sm(int tsdf_type, bool shade, bool color);
 // ingest: some slot's frame may be read in place (BatchTable::frame)
 void launch_filter(const BatchTable* bt, cudaStream_t st, int bil_rows = 8, bool ingest = false);
 void launch_input_maps(const BatchTable* bt, cudaStream_t st);
