@@ -11,8 +11,9 @@
 //   per block   warp-shuffle butterfly, then shared memory across warps
 //   per grid    the last block to finish an iteration (atomic ticket) sums
 //               the block partials in a fixed order, solves the 6x6 system in
-//               FP64 (LDL^T with the reference's failure rules,
-//               _yooji_cuda_math.h:489-592), tests convergence
+//               FP64 (elimination without divisions; the reference's failure
+//               rules, _yooji_cuda_math.h:489-592, from a float LDL^T beside
+//               it), tests convergence
 //               (|x|_inf < 5e-7, :971-972) and applies the SE(3) update in
 //               FP64 (T_12 <- exp(x) T_12, :976-978)
 //
@@ -571,8 +572,8 @@ __device__ void warp_rigid_inverse(const double* T, int lane, double& out) {
 // converged) costs nothing.  With one launch per iteration every iteration
 // paid the launch, the reads of the tables and the slowest session's closing
 // block: tracking of one 640x480 frame took 307 us in 19 launches and 242 when
-// this launch replaced them, with FP64 sums 603 and 440 (146 and 285 now, with
-// the closing and the lists below).
+// this launch replaced them, with FP64 sums 603 and 440 (148 and 255 now, with
+// the closing and the lists below; the kernel alone in each case).
 //
 // Progress needs no block but the running ones: a range is claimed only by a
 // block that then runs it, a closer goes on claiming ranges itself, and a
